@@ -1830,13 +1830,15 @@ int clb_voxelise_mesh(const float* triangles, uint8_t* mask, int triangle_count,
     CLB_REQUIRE(triangles != nullptr, "voxelise_mesh: null triangles");
     float d[3];
     voxelise_direction(d);
-    const dim3 grid((nz + VOX_BK - 1) / VOX_BK, (ny + VOX_BJ - 1) / VOX_BJ, (nx + VOX_BI - 1) / VOX_BI);
-    if (cull)
-        k_voxelise<true><<<grid, VOX_THREADS, 0, CLB_STREAM(stream)>>>(triangles, mask, triangle_count, nx, ny, nz,
+    if (cull) {
+        const dim3 grid((nz + VC_BK - 1) / VC_BK, (ny + VC_BJ - 1) / VC_BJ, (nx + VC_BI - 1) / VC_BI);
+        k_voxelise_culled<<<grid, VC_THREADS, 0, CLB_STREAM(stream)>>>(triangles, mask, triangle_count, nx, ny, nz,
                                                                        delta, ox, oy, oz, d[0], d[1], d[2]);
-    else
-        k_voxelise<false><<<grid, VOX_THREADS, 0, CLB_STREAM(stream)>>>(triangles, mask, triangle_count, nx, ny, nz,
-                                                                        delta, ox, oy, oz, d[0], d[1], d[2]);
+    } else {
+        const dim3 grid((nz + VOX_BK - 1) / VOX_BK, (ny + VOX_BJ - 1) / VOX_BJ, (nx + VOX_BI - 1) / VOX_BI);
+        k_voxelise_all<<<grid, VOX_THREADS, 0, CLB_STREAM(stream)>>>(triangles, mask, triangle_count, nx, ny, nz, delta,
+                                                                     ox, oy, oz, d[0], d[1], d[2]);
+    }
     CLB_LAUNCH_CHECK("k_voxelise");
     return 0;
 }
