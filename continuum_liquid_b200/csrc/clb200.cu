@@ -18,7 +18,7 @@
 #include "voxelise.cuh"
 #include "tc_gemm.cuh"
 #include "conv3d.cuh"
-#include "conv_win.cuh"
+#include "conv_march.cuh"
 
 #include <mutex>
 
@@ -74,8 +74,9 @@ static cudaError_t cluster_visit_attr() {
 }
 
 template <int N, bool DG>
-static cudaError_t conv_win_attr() {
-    return cudaFuncSetAttribute(conv::k_conv_win<N, DG>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+static cudaError_t conv_march_attr() {
+    return conv::conv_march_run<N, DG>(true, nullptr, nullptr, nullptr, nullptr, nullptr, conv::Vol{}, 0, 0, 0, false,
+                                       conv::MarchPlan{}, nullptr);
 }
 template <int N>
 static cudaError_t conv_wgrad_attr() {
@@ -84,14 +85,14 @@ static cudaError_t conv_wgrad_attr() {
 }
 static int conv_set_attributes() {
     cudaError_t e = cudaSuccess;
-    e = e != cudaSuccess ? e : conv_win_attr<16, false>();
-    e = e != cudaSuccess ? e : conv_win_attr<32, false>();
-    e = e != cudaSuccess ? e : conv_win_attr<64, false>();
-    e = e != cudaSuccess ? e : conv_win_attr<16, true>();
-    e = e != cudaSuccess ? e : conv_win_attr<32, true>();
-    e = e != cudaSuccess ? e : conv_win_attr<48, true>();
-    e = e != cudaSuccess ? e : conv_win_attr<64, true>();
-    e = e != cudaSuccess ? e : conv_win_attr<96, true>();
+    e = e != cudaSuccess ? e : conv_march_attr<16, false>();
+    e = e != cudaSuccess ? e : conv_march_attr<32, false>();
+    e = e != cudaSuccess ? e : conv_march_attr<64, false>();
+    e = e != cudaSuccess ? e : conv_march_attr<16, true>();
+    e = e != cudaSuccess ? e : conv_march_attr<32, true>();
+    e = e != cudaSuccess ? e : conv_march_attr<48, true>();
+    e = e != cudaSuccess ? e : conv_march_attr<64, true>();
+    e = e != cudaSuccess ? e : conv_march_attr<96, true>();
     e = e != cudaSuccess ? e : conv_wgrad_attr<16>();
     e = e != cudaSuccess ? e : conv_wgrad_attr<32>();
     e = e != cudaSuccess ? e : conv_wgrad_attr<64>();
@@ -1609,21 +1610,20 @@ int clb_conv3d_forward(const void* x, const void* wf, const float* bias, void* y
     CLB_REQUIRE(kpad % 64 == 0 && kpad >= 27 * cin, "conv3d_forward: kpad=%d must be a multiple of 64 >= 27*cin", kpad);
     CLB_REQUIRE(cout == 16 || cout == 32 || cout == 64, "conv3d_forward: cout=%d not supported (16, 32, 64)", cout);
     CLB_REQUIRE(bias == nullptr || ((uintptr_t)bias & 15) == 0, "conv3d_forward: bias must be 16-byte aligned");
-    conv::WinPlan pl;
-    CLB_REQUIRE(conv::win_plan(D, H, W, cin, cout, B, pl), "conv3d_forward: no block shape fits %dx%dx%d", D, H, W);
+    conv::MarchPlan pl;
+    CLB_REQUIRE(conv::march_plan(B, D, H, W, cin, cout, cin == 8, g_sm_count, pl), "conv3d_forward: no block shape fits %dx%dx%d", D, H, W);
     const conv::Vol g{B, D, H, W};
-    const unsigned blocks = (unsigned)((i64)B * D * pl.ytiles * pl.xtiles);
     cudaStream_t s = CLB_STREAM(stream);
     const auto* X = (const __nv_bfloat16*)x;
     const auto* Wf = (const __nv_bfloat16*)wf;
     auto* Y = (__nv_bfloat16*)y;
 #define CLB_FW(NN) \
-    conv::k_conv_win<NN, false><<<blocks, conv::CW_THREADS, pl.smem, s>>>(X, Wf, bias, nullptr, Y, g, cin, kpad, relu, pl)
+    (void)conv::conv_march_run<NN, false>(false, X, Wf, bias, nullptr, Y, g, cin, kpad, relu, cin == 8, pl, s)
     if (cout == 16) CLB_FW(16);
     else if (cout == 32) CLB_FW(32);
     else CLB_FW(64);
 #undef CLB_FW
-    CLB_LAUNCH_CHECK("k_conv_win<forward>");
+    CLB_LAUNCH_CHECK("k_conv_march<forward>");
     return 0;
 }
 
@@ -1635,24 +1635,23 @@ int clb_conv3d_dgrad(const void* dy, const void* wd, const void* mask_x, void* d
     CLB_REQUIRE(kpad % 64 == 0 && kpad >= 27 * cout, "conv3d_dgrad: kpad=%d must be a multiple of 64 >= 27*cout", kpad);
     CLB_REQUIRE(cin == 16 || cin == 32 || cin == 48 || cin == 64 || cin == 96,
                 "conv3d_dgrad: cin=%d not supported (16, 32, 48, 64, 96)", cin);
-    conv::WinPlan pl;
-    CLB_REQUIRE(conv::win_plan(D, H, W, cout, cin, B, pl), "conv3d_dgrad: no block shape fits %dx%dx%d", D, H, W);
+    conv::MarchPlan pl;
+    CLB_REQUIRE(conv::march_plan(B, D, H, W, cout, cin, false, g_sm_count, pl), "conv3d_dgrad: no block shape fits %dx%dx%d", D, H, W);
     const conv::Vol g{B, D, H, W};
-    const unsigned blocks = (unsigned)((i64)B * D * pl.ytiles * pl.xtiles);
     cudaStream_t s = CLB_STREAM(stream);
     const auto* DY = (const __nv_bfloat16*)dy;
     const auto* Wd = (const __nv_bfloat16*)wd;
     const auto* MX = (const __nv_bfloat16*)mask_x;
     auto* DX = (__nv_bfloat16*)dx;
 #define CLB_DG(NN) \
-    conv::k_conv_win<NN, true><<<blocks, conv::CW_THREADS, pl.smem, s>>>(DY, Wd, nullptr, MX, DX, g, cout, kpad, 0, pl)
+    (void)conv::conv_march_run<NN, true>(false, DY, Wd, nullptr, MX, DX, g, cout, kpad, 0, false, pl, s)
     if (cin == 16) CLB_DG(16);
     else if (cin == 32) CLB_DG(32);
     else if (cin == 48) CLB_DG(48);
     else if (cin == 64) CLB_DG(64);
     else CLB_DG(96);
 #undef CLB_DG
-    CLB_LAUNCH_CHECK("k_conv_win<dgrad>");
+    CLB_LAUNCH_CHECK("k_conv_march<dgrad>");
     return 0;
 }
 

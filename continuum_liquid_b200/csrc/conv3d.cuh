@@ -1,12 +1,12 @@
 // 3x3x3 convolutions (padding 1, stride 1) of the learned pressure warm start as implicit GEMMs on
-// the tcgen05 core (tc_gemm.cuh). Activations are channels-last BF16 volumes [B][D][H][W][C] with C a
+// tcgen05. Activations are channels-last BF16 volumes [B][D][H][W][C] with C a
 // multiple of 8; the 27 taps are ordered (dz, dy, dx) with dx fastest, offsets -1..1.
 //
 //   forward   y[v][co] = act(b[co] + sum_{tap,ci} x[v + o(tap)][ci] * W[tap][ci][co])
-//             GEMM: M = voxels (tiles of 128), N = Cout, K = 27 * Cin (K-major gathers of x, weights
-//             pre-arranged as wf[co][tap * Cin + ci]); bias and ReLU fused in the epilogue.
+//             GEMM: M = voxels, N = Cout, K = 27 * Cin (conv_march.cuh; weights pre-arranged as
+//             wf[co][tap * Cin + ci]); bias and ReLU fused in the epilogue.
 //   data grad dx[v][ci] = mask(ci) * sum_{tap,co} dy[v - o(tap)][co] * W[tap][ci][co]
-//             GEMM: M = voxels, N = Cin, K = 27 * Cout (wd[ci][tap * Cout + co]); the ReLU backward
+//             GEMM: M = voxels, N = Cin, K = 27 * Cout (the same kernel, wd[ci][tap * Cout + co]); the ReLU backward
 //             of the layer that produced x (mask = x > 0) is fused in the epilogue.
 //   weight grad dW[tap * Cin + ci][co] += sum_v x[v + o(tap)][ci] * dy[v][co]
 //             GEMM: M = 27 * Cin (tiles of 128), N = Cout, K = voxels split over blocks; both
@@ -47,99 +47,6 @@ __device__ __forceinline__ void decode(const Vol& g, int v, int& b, int& z, int&
 __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<const uint32_t*>(&h);
-}
-
-// ---- forward and data gradient: A = gathered activations (K-major), B = arranged weights ----------
-template <int N, bool DGRAD>
-struct ConvRows {
-    static constexpr bool A_MN = false, B_MN = false;
-    const __nv_bfloat16* src;  // forward: x [V][Cs]; data grad: dy [V][Cs]
-    const __nv_bfloat16* wmat;  // [N][Kpad] bf16
-    const float* bias;          // forward only (nullable)
-    const __nv_bfloat16* mask_src;  // data grad: x [V][N] for the ReLU mask (nullable)
-    __nv_bfloat16* out;         // [V][N]
-    Vol g;
-    int Cs, K, Kpad, chunks, m0, relu;
-    int vb, vz, vy, vx;  // this thread's row voxel (row = threadIdx.x)
-    bool valid;
-    __device__ void setup() {
-        const int v = m0 + threadIdx.x;
-        valid = v < g.voxels();
-        if (valid) decode(g, v, vb, vz, vy, vx);
-    }
-    __device__ void gather_a(uint8_t* st, int chunk) const {
-        const int row = threadIdx.x;
-#pragma unroll
-        for (int kv = 0; kv < TC_KC / 8; ++kv) {
-            const int k = chunk * TC_KC + kv * 8;
-            uint4 val = make_uint4(0, 0, 0, 0);
-            if (valid && k < K) {
-                const int tap = k / Cs, c = k - tap * Cs;
-                const int nb = tap_neighbour(g, vb, vz, vy, vx, tap, DGRAD ? -1 : 1);
-                if (nb >= 0) val = __ldg(reinterpret_cast<const uint4*>(src + (i64)nb * Cs + c));
-            }
-            *reinterpret_cast<uint4*>(st + tc::kmajor_off(row, kv)) = val;
-        }
-    }
-    __device__ void gather_b(uint8_t* st, int chunk) const {
-        for (int t = threadIdx.x; t < N * (TC_KC / 8); t += TC_THREADS) {
-            const int row = t / (TC_KC / 8), kv = t % (TC_KC / 8);
-            const uint4 val = __ldg(reinterpret_cast<const uint4*>(wmat + (i64)row * Kpad + chunk * TC_KC + kv * 8));
-            *reinterpret_cast<uint4*>(st + tc::kmajor_off(row, kv)) = val;
-        }
-    }
-    __device__ void epilogue(int row, const float* acc, int col0) const {
-        const int v = m0 + row;
-        if (v >= g.voxels()) return;
-        float r[16];
-#pragma unroll
-        for (int q = 0; q < 16; ++q) {
-            float a = acc[q];
-            if (!DGRAD) {
-                if (bias) a += __ldg(bias + col0 + q);
-                if (relu) a = fmaxf(a, 0.0f);
-            }
-            r[q] = a;
-        }
-        if (DGRAD && mask_src) {
-            const uint4* m4 = reinterpret_cast<const uint4*>(mask_src + (i64)v * N + col0);
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const uint4 mv = __ldg(m4 + h);
-                const __nv_bfloat16* mb = reinterpret_cast<const __nv_bfloat16*>(&mv);
-#pragma unroll
-                for (int q = 0; q < 8; ++q)
-                    if (!(__bfloat162float(mb[q]) > 0.0f)) r[8 * h + q] = 0.0f;
-            }
-        }
-        uint4* o4 = reinterpret_cast<uint4*>(out + (i64)v * N + col0);
-        o4[0] = make_uint4(pack_bf16x2(r[0], r[1]), pack_bf16x2(r[2], r[3]), pack_bf16x2(r[4], r[5]),
-                           pack_bf16x2(r[6], r[7]));
-        o4[1] = make_uint4(pack_bf16x2(r[8], r[9]), pack_bf16x2(r[10], r[11]), pack_bf16x2(r[12], r[13]),
-                           pack_bf16x2(r[14], r[15]));
-    }
-};
-
-template <int N, bool DGRAD>
-__global__ void __launch_bounds__(TC_THREADS) k_conv_rows(const __nv_bfloat16* src, const __nv_bfloat16* wmat,
-                                                           const float* bias, const __nv_bfloat16* mask_src,
-                                                           __nv_bfloat16* out, Vol g, int Cs, int Kpad, int relu) {
-    extern __shared__ __align__(1024) uint8_t smem[];
-    ConvRows<N, DGRAD> op;
-    op.src = src;
-    op.wmat = wmat;
-    op.bias = bias;
-    op.mask_src = mask_src;
-    op.out = out;
-    op.g = g;
-    op.Cs = Cs;
-    op.K = 27 * Cs;
-    op.Kpad = Kpad;
-    op.chunks = Kpad / TC_KC;
-    op.m0 = blockIdx.x * TC_M;
-    op.relu = relu;
-    op.setup();
-    tc::tile_gemm<ConvRows<N, DGRAD>, N>(op, smem);
 }
 
 // ---- weight gradient: A = x at tap offsets (MN-major over (tap, ci)), B = dy (MN-major over co) ---
