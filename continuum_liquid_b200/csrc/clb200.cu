@@ -19,6 +19,7 @@
 #include "tc_gemm.cuh"
 #include "conv3d.cuh"
 #include "conv_march.cuh"
+#include "conv_wgrad.cuh"
 
 #include <mutex>
 
@@ -78,10 +79,10 @@ static cudaError_t conv_march_attr() {
     return conv::conv_march_run<N, DG>(true, nullptr, nullptr, nullptr, nullptr, nullptr, conv::Vol{}, 0, 0, 0, false,
                                        conv::MarchPlan{}, nullptr);
 }
-template <int N>
+template <int NC>
 static cudaError_t conv_wgrad_attr() {
-    return cudaFuncSetAttribute(conv::k_conv_wgrad<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)tc::tile_smem_bytes<N>());
+    return cudaFuncSetAttribute(conv::k_conv_wgrad_march<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                conv::CM_SMEM_LIMIT);
 }
 static int conv_set_attributes() {
     cudaError_t e = cudaSuccess;
@@ -95,7 +96,6 @@ static int conv_set_attributes() {
     e = e != cudaSuccess ? e : conv_march_attr<96, true>();
     e = e != cudaSuccess ? e : conv_wgrad_attr<16>();
     e = e != cudaSuccess ? e : conv_wgrad_attr<32>();
-    e = e != cudaSuccess ? e : conv_wgrad_attr<64>();
     return check_call(e, "convolution attributes");
 }
 
@@ -1661,22 +1661,19 @@ int clb_conv3d_wgrad(const void* x, const void* dy, float* dw, int B, int D, int
     CLB_REQUIRE(x && dy && dw, "conv3d_wgrad: null pointer");
     CLB_REQUIRE(cin > 0 && cin % 8 == 0, "conv3d_wgrad: cin=%d must be a positive multiple of 8", cin);
     CLB_REQUIRE(chunks_per_block > 0, "conv3d_wgrad: chunks_per_block must be positive");
+    CLB_REQUIRE(cout == 16 || cout == 32 || cout == 64, "conv3d_wgrad: cout=%d not supported (16, 32, 64)", cout);
+    conv::WgradPlan pl;
+    CLB_REQUIRE(conv::wgrad_plan(B, D, H, W, cin, cout, chunks_per_block, ((uintptr_t)dw & 15) == 0, g_sm_count, pl),
+                "conv3d_wgrad: no block shape fits %dx%dx%d", D, H, W);
     const conv::Vol g{B, D, H, W};
-    const i64 chunks = ((i64)B * D * H * W + tc::TC_KC - 1) / tc::TC_KC;
-    const dim3 grid((unsigned)((27 * cin + tc::TC_M - 1) / tc::TC_M),
-                    (unsigned)((chunks + chunks_per_block - 1) / chunks_per_block));
     cudaStream_t s = CLB_STREAM(stream);
     const auto* X = (const __nv_bfloat16*)x;
     const auto* DY = (const __nv_bfloat16*)dy;
     if (cout == 16)
-        conv::k_conv_wgrad<16><<<grid, tc::TC_THREADS, tc::tile_smem_bytes<16>(), s>>>(X, DY, dw, g, cin, chunks_per_block);
-    else if (cout == 32)
-        conv::k_conv_wgrad<32><<<grid, tc::TC_THREADS, tc::tile_smem_bytes<32>(), s>>>(X, DY, dw, g, cin, chunks_per_block);
-    else if (cout == 64)
-        conv::k_conv_wgrad<64><<<grid, tc::TC_THREADS, tc::tile_smem_bytes<64>(), s>>>(X, DY, dw, g, cin, chunks_per_block);
+        conv::k_conv_wgrad_march<16><<<pl.grid, conv::WG_THREADS, pl.smem, s>>>(X, DY, dw, g, cin, cout, pl);
     else
-        return set_error("conv3d_wgrad: cout=%d not supported (16, 32, 64)", cout);
-    CLB_LAUNCH_CHECK("k_conv_wgrad");
+        conv::k_conv_wgrad_march<32><<<pl.grid, conv::WG_THREADS, pl.smem, s>>>(X, DY, dw, g, cin, cout, pl);
+    CLB_LAUNCH_CHECK("k_conv_wgrad_march");
     return 0;
 }
 
@@ -1757,8 +1754,9 @@ int clb_unet_head_backward(const void* h, const float* w, const float* dout, voi
 
 int clb_unet_bias_grad(const void* dy, float* db, int voxels, int C, void* stream) {
     CLB_REQUIRE(C > 0 && C <= 256 && C % 8 == 0, "unet_bias_grad: C=%d must be a multiple of 8 in 8..256", C);
-    conv::k_bias_grad<<<ew_blocks((i64)voxels * C / 16), conv::EW, 0, CLB_STREAM(stream)>>>((const __nv_bfloat16*)dy, db,
-                                                                                            voxels, C);
+    const unsigned wanted = ew_blocks((i64)voxels * C / 32);  // four voxel groups a thread
+    conv::k_bias_grad<<<wanted < conv::BG_BLOCKS ? wanted : conv::BG_BLOCKS, conv::EW, 0, CLB_STREAM(stream)>>>(
+        (const __nv_bfloat16*)dy, db, voxels, C);
     CLB_LAUNCH_CHECK("k_bias_grad");
     return 0;
 }

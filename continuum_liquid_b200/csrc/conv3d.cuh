@@ -9,9 +9,8 @@
 //             GEMM: M = voxels, N = Cin, K = 27 * Cout (the same kernel, wd[ci][tap * Cout + co]); the ReLU backward
 //             of the layer that produced x (mask = x > 0) is fused in the epilogue.
 //   weight grad dW[tap * Cin + ci][co] += sum_v x[v + o(tap)][ci] * dy[v][co]
-//             GEMM: M = 27 * Cin (tiles of 128), N = Cout, K = voxels split over blocks; both
-//             operands MN-major (16-byte rows of 8 consecutive channels); FP32 atomics in the
-//             epilogue accumulate the blocks' partial sums.
+//             GEMM: K = voxels split over blocks, both operands MN-major, the taps from addresses
+//             (conv_wgrad.cuh); FP32 reductions add the blocks' partial sums.
 #pragma once
 #include "tc_gemm.cuh"
 
@@ -47,68 +46,6 @@ __device__ __forceinline__ void decode(const Vol& g, int v, int& b, int& z, int&
 __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<const uint32_t*>(&h);
-}
-
-// ---- weight gradient: A = x at tap offsets (MN-major over (tap, ci)), B = dy (MN-major over co) ---
-template <int N>
-struct ConvWgrad {
-    static constexpr bool A_MN = true, B_MN = true;
-    const __nv_bfloat16* x;   // [V][Cin]
-    const __nv_bfloat16* dy;  // [V][N]
-    float* dw;                // [27 * Cin][N], accumulated
-    Vol g;
-    int Cin, Mrows, m0, chunk0, chunks;
-    __device__ void gather_a(uint8_t* st, int chunk) const {
-        const int kk = threadIdx.x & (TC_KC - 1);
-        const int v = (chunk0 + chunk) * TC_KC + kk;
-        int b = 0, z = 0, y = 0, xx = 0;
-        const bool valid = v < g.voxels();
-        if (valid) decode(g, v, b, z, y, xx);
-        for (int mv = threadIdx.x / TC_KC; mv < TC_M / 8; mv += TC_THREADS / TC_KC) {
-            const int m = m0 + mv * 8;
-            uint4 val = make_uint4(0, 0, 0, 0);
-            if (valid && m < Mrows) {
-                const int tap = m / Cin, c = m - tap * Cin;
-                const int nb = tap_neighbour(g, b, z, y, xx, tap, 1);
-                if (nb >= 0) val = __ldg(reinterpret_cast<const uint4*>(x + (i64)nb * Cin + c));
-            }
-            *reinterpret_cast<uint4*>(st + tc::mnmajor_off(mv, kk)) = val;
-        }
-    }
-    __device__ void gather_b(uint8_t* st, int chunk) const {
-        const int kk = threadIdx.x & (TC_KC - 1);
-        const int v = (chunk0 + chunk) * TC_KC + kk;
-        const bool valid = v < g.voxels();
-        for (int nv = threadIdx.x / TC_KC; nv < N / 8; nv += TC_THREADS / TC_KC) {
-            uint4 val = make_uint4(0, 0, 0, 0);
-            if (valid) val = __ldg(reinterpret_cast<const uint4*>(dy + (i64)v * N + nv * 8));
-            *reinterpret_cast<uint4*>(st + tc::mnmajor_off(nv, kk)) = val;
-        }
-    }
-    __device__ void epilogue(int row, const float* acc, int col0) const {
-        const int m = m0 + row;
-        if (m >= Mrows) return;
-#pragma unroll
-        for (int q = 0; q < 16; ++q) atomicAdd(dw + (i64)m * N + col0 + q, acc[q]);
-    }
-};
-
-template <int N>
-__global__ void __launch_bounds__(TC_THREADS) k_conv_wgrad(const __nv_bfloat16* x, const __nv_bfloat16* dy,
-                                                            float* dw, Vol g, int Cin, int chunks_per_block) {
-    extern __shared__ __align__(1024) uint8_t smem[];
-    ConvWgrad<N> op;
-    op.x = x;
-    op.dy = dy;
-    op.dw = dw;
-    op.g = g;
-    op.Cin = Cin;
-    op.Mrows = 27 * Cin;
-    op.m0 = blockIdx.x * TC_M;
-    const int total_chunks = (g.B * g.D * g.H * g.W + TC_KC - 1) / TC_KC;
-    op.chunk0 = blockIdx.y * chunks_per_block;
-    op.chunks = max(0, min(chunks_per_block, total_chunks - op.chunk0));
-    tc::tile_gemm<ConvWgrad<N>, N>(op, smem);
 }
 
 // ---- elementwise pieces of the network ------------------------------------------------------------
@@ -329,8 +266,13 @@ __global__ void k_head_backward(const __nv_bfloat16* __restrict__ h, const float
 }
 
 // bias gradient of a conv: db[co] += sum_v dy[v][co]. Thread t of a block sums channel group
-// t % G (8 channels) over voxels t / G, t / G + stride, ... (blockDim is a multiple of G).
-__global__ void k_bias_grad(const __nv_bfloat16* __restrict__ dy, float* db, int V, int C) {
+// t % G (8 channels) over voxels t / G, t / G + stride, ... (blockDim is a multiple of G when G is a power of two).
+// Bound by reading dy once; what cost more was the end of each of many short blocks, 256 threads adding to the same C
+// shared-memory words. So few blocks (BG_BLOCKS) walk the voxels with four loads in flight, and lanes of one
+// channel group first add up by shuffles when G is a power of two. 2.1M voxels of 16 channels: 131 -> 10 us.
+constexpr int BG_BLOCKS = 148 * 3;
+
+__global__ void __launch_bounds__(256) k_bias_grad(const __nv_bfloat16* __restrict__ dy, float* db, int V, int C) {
     __shared__ float s[256];
     const int G = C / 8;
     for (int c = threadIdx.x; c < C; c += blockDim.x) s[c] = 0.0f;
@@ -338,16 +280,38 @@ __global__ void k_bias_grad(const __nv_bfloat16* __restrict__ dy, float* db, int
     const int per_block = blockDim.x / G;
     const int grp = threadIdx.x % G, slot = threadIdx.x / G;
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    if (slot < per_block)
-        for (i64 v = (i64)blockIdx.x * per_block + slot; v < V; v += (i64)gridDim.x * per_block) {
+    if (slot < per_block) {
+        const i64 stride = (i64)gridDim.x * per_block;
+        const uint4* src = reinterpret_cast<const uint4*>(dy) + grp;
+        i64 v = (i64)blockIdx.x * per_block + slot;
+        for (; v + 3 * stride < V; v += 4 * stride) {
+            uint4 u[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) u[q] = __ldg(src + (v + q * stride) * G);
+            float f[4][8];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) unpack8(u[q], f[q]);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) acc[e] += (f[0][e] + f[1][e]) + (f[2][e] + f[3][e]);
+        }
+        for (; v < V; v += stride) {
             float f[8];
-            unpack8(__ldg(reinterpret_cast<const uint4*>(dy + v * C) + grp), f);
+            unpack8(__ldg(src + v * G), f);
 #pragma unroll
             for (int e = 0; e < 8; ++e) acc[e] += f[e];
         }
-    if (slot < per_block)
+    }
+    if ((G & (G - 1)) == 0 && G <= 32) {  // uniform: every thread has a slot
+        for (int o = 16; o >= G; o >>= 1)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
+        if ((threadIdx.x & 31) < G)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) atomicAdd(&s[grp * 8 + e], acc[e]);
+    } else if (slot < per_block) {
 #pragma unroll
         for (int e = 0; e < 8; ++e) atomicAdd(&s[grp * 8 + e], acc[e]);
+    }
     __syncthreads();
     for (int c = threadIdx.x; c < C; c += blockDim.x) atomicAdd(db + c, s[c]);
 }
