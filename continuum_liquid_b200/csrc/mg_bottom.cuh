@@ -12,6 +12,15 @@
 // neighbour weights of A cells are read from shared memory, those of B cells are registers too). The
 // update formula and every summation order are those of multigrid.cl (rbgs_step, restrict_residual,
 // prolongate), so the result is identical to the launch-per-kernel W-cycle.
+//
+// What bounds a visit is the latency of B's dependent phases (264 a visit with the reference's counts): a barrier,
+// six shared-memory loads, a chain of five additions, a division and a store. So a phase is kept short:
+//   * only as many warps as hold fluid cells of B take part, one cell of a colour per thread as long as 16 warps
+//     suffice (a second cell costs a thread 50-90 cycles, another warp 2-6), and one warp needs no barrier;
+//   * B's p lies split by colour (split_cell): consecutive words per phase instead of every second one;
+//   * the addresses of a cell's six neighbours are registers, and the division is divide_by.
+// Cycles of a phase (B200, 25 / 256 / 512 cells of a colour): 151 / 186 / 240; with 8 warps throughout, up to two
+// cells a thread, unsplit rows and the general division 211 / 224 / 384.
 #pragma once
 #include "multigrid.cuh"
 
@@ -19,7 +28,7 @@ namespace clb {
 
 constexpr int BOTTOM_THREADS = 512;
 constexpr int BOTTOM_MAX_A = 8;  // A slots of each colour per thread
-constexpr int BOTTOM_MAX_B = 4;  // B slots of each colour per B thread
+constexpr int BOTTOM_MAX_B = 4;  // B slots of each colour per 256 threads
 
 static inline size_t bottom_smem_bytes(int ca, int cb) {
     // A: p, b, op(float4); B: p, op(float4); the fluid-cell lists of both colours of both levels and
@@ -49,26 +58,50 @@ __device__ __forceinline__ int colour_cell(int r, int colour, int nx, int ny, in
     return (i * ny + j) * nz + k;
 }
 
+// x / d for a positive integer-valued d up to 32768 (every diagonal: a sum of small weights) with r = 1 / d correctly
+// rounded: Markstein's correction (P. Markstein, IBM J. Res. Dev. 34, 1990) of the product q = x r by its exact
+// remainder x - q d. Four dependent operations after x, without a branch, instead of the general division's dozen.
+// Correctly rounded for every significand and every such d (checked exhaustively) where |x| >= 2^-111; below, where
+// the remainder is no longer exact, the last bit of a subnormal quotient may differ. Infinities and NaN as x / d;
+// a zero quotient is +0.
+__device__ __forceinline__ float divide_by(float x, float d, float r) {
+    const float q = x * r;
+    const float y = __fmaf_rn(__fmaf_rn(-q, d, x), r, q);
+    return fabsf(x) < __int_as_float(0x7f800000) ? y : q;
+}
+
+// B's p in shared memory: cells of one colour together, rows of half = (nz - 1) / 2 slots (those of the
+// interior; rows of the ghost layer exist and hold 0), colour 0 first, after one word that always holds 0
+// (what neighbours in the ghost layer along k read). Never more words than the level has cells. All six
+// neighbours of a cell are of the other colour: along i and j in the same slot of other rows, along k in
+// slots s + t - 1 and s + t of its own row, t = (k - 1) & 1.
+__device__ __forceinline__ int split_cell(int i, int j, int k, int nx, int ny, int nz) {
+    const int half = (nz - 1) / 2;
+    return 1 + (((i + j + k) & 1) * nx * ny + i * ny + j) * half + ((k - 1) >> 1);
+}
+
 // Constants of one owned cell of the second-coarsest level: smem index, diagonal (<= 0: not updated;
 // -1 marks cells that are not fluid or slots without a cell) and delta^2 * b.
 struct OwnedCell {
     int c;
     float d;
+    float r;  // 1 / d
     float d2b;
 };
 
 // Owned coarsest-level cell with its neighbour weights in registers (constant for the whole visit).
 struct OwnedCellW {
-    int c;
-    float d, d2b;
+    int c, n;    // split_cell of the cell, and its slot in the other colour
+    int zp, zm;  // split cells of its neighbours along k
+    float d, r, d2b;
     float wxp, wxm, wyp, wym, wzp, wzm;
 };
 
-__device__ __forceinline__ void relax_w(const OwnedCellW& o, float* sp, int sx, int sy) {
-    const int c = o.c;
-    const float ws = o.wxp * sp[c + sx] + o.wxm * sp[c - sx] + o.wyp * sp[c + sy] + o.wym * sp[c - sy] +
-                     o.wzp * sp[c + 1] + o.wzm * sp[c - 1];
-    sp[c] = (ws - o.d2b) / o.d;
+// sx, sy: split-layout strides along i and j.
+__device__ __forceinline__ float relaxed_w(const OwnedCellW& o, const float* sp, int sx, int sy) {
+    const float ws = o.wxp * sp[o.n + sx] + o.wxm * sp[o.n - sx] + o.wyp * sp[o.n + sy] + o.wym * sp[o.n - sy] +
+                     o.wzp * sp[o.zp] + o.wzm * sp[o.zm];
+    return divide_by(ws - o.d2b, o.d, o.r);
 }
 
 // One red-black update of an owned cell (multigrid.cl:225-229), p and weights in shared memory.
@@ -77,15 +110,20 @@ __device__ __forceinline__ void relax(const OwnedCell& o, float* sp, const float
     const float4 self = so[c];
     const float ws = self.y * sp[c + sx] + so[c - sx].y * sp[c - sx] + self.z * sp[c + sy] + so[c - sy].z * sp[c - sy] +
                      self.w * sp[c + 1] + so[c - 1].w * sp[c - 1];
-    sp[c] = (ws - o.d2b) / o.d;
+    sp[c] = divide_by(ws - o.d2b, o.d, o.r);
 }
 
-// The coarsest level B runs on BOTTOM_BTHREADS threads (8 warps) that synchronise with a named
-// barrier; each owns slots r = thread, thread + 256, ... of both colours, so every thread updates
-// its cells of one colour per phase.
+// The coarsest level B: thread t owns the fluid cells t, t + 512 of either colour (bottom_lists), so the first
+// warps own them all, and those synchronise with a named barrier. BOTTOM_BTHREADS is what a plan counts B's
+// slots by (KB slots per 256 threads: BOTTOM_KB cells of a colour per thread here).
 constexpr int BOTTOM_BTHREADS = 256;
+__host__ __device__ constexpr int bottom_kb(int KB) { return (KB + 1) / 2; }
 
-__device__ __forceinline__ void bar_b() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+// Phases of B: warps 0 .. warps - 1 take part.
+__device__ __forceinline__ void bar_b(int warps) {
+    if (warps > 1) asm volatile("bar.sync 1, %0;" ::"r"(32 * warps) : "memory");
+    else __syncwarp();
+}
 
 // Shared-memory arrays of a bottom visit: A's p, b and operator (float4, diagonal -1 where not
 // fluid), B's p and operator, and the fluid cells of each colour of both levels; each region padded to
@@ -210,7 +248,7 @@ __device__ __forceinline__ void bottom_stage(const BottomSmem& S, const float* _
 template <int KA, int KB>
 struct BottomCells {
     OwnedCell A[2][KA];   // [colour][m]: the thread's fluid cells (bottom_lists)
-    OwnedCellW B[2][KB];  // [colour][m]
+    OwnedCellW B[2][bottom_kb(KB)];  // [colour][m]
 };
 
 // After the lists are built and the block has synchronised.
@@ -228,24 +266,31 @@ __device__ __forceinline__ void bottom_cells(const BottomSmem& S, BottomCells<KA
             OwnedCell& o = R.A[colour][m];
             o.c = c < 0 ? 0 : c;
             o.d = c < 0 ? -1.0f : S.soa[c].x;  // fluid: >= 0
+            o.r = 1.0f / o.d;
             o.d2b = 0.0f;
         }
-    const bool btile = threadIdx.x < BOTTOM_BTHREADS;
 #pragma unroll
     for (int colour = 0; colour < 2; ++colour)
 #pragma unroll
-        for (int m = 0; m < KB; ++m) {
-            const int r = threadIdx.x + m * BOTTOM_BTHREADS;
-            const int c = btile && r < S.count[2 + colour] ? S.list_b[colour * lb + r] : -1;
+        for (int m = 0; m < bottom_kb(KB); ++m) {
+            const int r = threadIdx.x + m * BOTTOM_THREADS;
+            const int c = r < S.count[2 + colour] ? S.list_b[colour * lb + r] : -1;
             OwnedCellW& o = R.B[colour][m];
             o.d2b = 0.0f;
-            o.c = 0;
-            o.d = -1.0f;
+            o.c = o.zp = o.zm = 0;
+            o.n = 1 + bny * ((bnz - 1) / 2);  // a slot without a cell loads some cells and stores nothing
+            o.d = o.r = -1.0f;
             o.wxp = o.wxm = o.wyp = o.wym = o.wzp = o.wzm = 0.0f;
             if (c >= 0) {
                 const float4 self = S.sob[c];
-                o.c = c;
+                const int i = c / bsx, j = (c / bsy) % bny, k = c % bnz;
+                o.c = split_cell(i, j, k, bnx, bny, bnz);
+                o.n = o.c + (((i + j + k) & 1) ? -1 : 1) * bnx * bny * ((bnz - 1) / 2);
+                const int up = o.n + ((k - 1) & 1);
+                o.zp = k + 1 <= bnz - 2 ? up : 0;
+                o.zm = k > 1 ? up - 1 : 0;
                 o.d = self.x;
+                o.r = 1.0f / o.d;
                 o.wxp = self.y;
                 o.wyp = self.z;
                 o.wzp = self.w;
@@ -271,7 +316,7 @@ __device__ __forceinline__ void bottom_rhs(const BottomSmem& S, BottomCells<KA, 
 // One visit of A from staged shared memory with the owned cells set (bottom_cells, bottom_rhs):
 // pre-smoothing of A, restriction into B (B's p zeroed, multigrid.cl:114), the two coarse solves of B,
 // prolongation, post-smoothing of A. bb (nullable): B's right-hand side is stored there (FP16 when H).
-// KA: A slots of each colour per thread (of BOTTOM_THREADS); KB: B slots of each colour per B thread.
+// KA: A slots of each colour per thread (of BOTTOM_THREADS); KB: B slots of each colour per 256 threads.
 template <int KA, int KB, bool H>
 __device__ __forceinline__ void bottom_core(const BottomSmem& S, BottomCells<KA, KB>& R, int anx, int any, int anz,
                                             int bnx, int bny, int bnz, float d2, float inv_delta2, int pre, int post,
@@ -287,10 +332,11 @@ __device__ __forceinline__ void bottom_core(const BottomSmem& S, BottomCells<KA,
         else a[c] = v;
     };
     const int asx = any * anz, asy = anz, bsx = bny * bnz, bsy = bnz;
+    const int half = (bnz - 1) / 2;  // split-layout strides: bny * half along i, half along j
     const int lb = CB / 2 + 1;
+    constexpr int MB = bottom_kb(KB);
     OwnedCell (&A)[2][KA] = R.A;
-    OwnedCellW (&B)[2][KB] = R.B;
-    const bool btile = threadIdx.x < BOTTOM_BTHREADS;
+    OwnedCellW (&B)[2][MB] = R.B;
 
     auto smooth_a = [&](int iterations) {
         for (int it = 0; it < iterations; ++it)
@@ -337,15 +383,15 @@ __device__ __forceinline__ void bottom_core(const BottomSmem& S, BottomCells<KA,
 #pragma unroll
             for (int l = 0; l < 8; ++l)
                 if (present[l]) rhs += r[l];
-            spb[cb] = rhs;
+            spb[split_cell(I, J, K, bnx, bny, bnz)] = rhs;
         }
     }
     __syncthreads();
-    float bvals[2][KB];
+    float bvals[2][MB];
 #pragma unroll
     for (int colour = 0; colour < 2; ++colour)
 #pragma unroll
-        for (int m = 0; m < KB; ++m) {
+        for (int m = 0; m < MB; ++m) {
             // a fluid cell (slots without a cell and air cells hold -1)
             const float rhs = B[colour][m].d >= 0.0f ? spb[B[colour][m].c] : 0.0f;
             bvals[colour][m] = rhs;
@@ -354,17 +400,22 @@ __device__ __forceinline__ void bottom_core(const BottomSmem& S, BottomCells<KA,
     __syncthreads();
     for (int c = threadIdx.x; c < CB; c += BOTTOM_THREADS) spb[c] = 0.0f;  // multigrid.cl:114
     __syncthreads();
-    if (btile) {
+    const int most = max(S.count[2], S.count[3]);
+    const int bwarps = min(BOTTOM_THREADS / 32, (most + 31) / 32);
+    if ((int)(threadIdx.x >> 5) < bwarps) {
         // two coarse solves of the W (multigrid.py:127-170; b_solves: one when the coarsest level is
         // visited once), pre + coarse_iters iterations each
-        const int iterations = b_solves * (pre + coarse_iters);
+        const int iterations = b_solves * (pre + coarse_iters), sx = bny * half, sy = half;
         for (int it = 0; it < iterations; ++it)
 #pragma unroll
             for (int colour = 0; colour < 2; ++colour) {
+                float v[MB];
 #pragma unroll
-                for (int m = 0; m < KB; ++m)
-                    if (B[colour][m].d > 0.0f) relax_w(B[colour][m], spb, bsx, bsy);
-                bar_b();
+                for (int m = 0; m < MB; ++m) v[m] = relaxed_w(B[colour][m], spb, sx, sy);
+#pragma unroll
+                for (int m = 0; m < MB; ++m)
+                    if (B[colour][m].d > 0.0f) spb[B[colour][m].c] = v[m];
+                bar_b(bwarps);
             }
     }
     __syncthreads();
@@ -378,7 +429,7 @@ __device__ __forceinline__ void bottom_core(const BottomSmem& S, BottomCells<KA,
             const int i = c / asx, j = (c / asy) % any, k = c % anz;
             const int I = min((i - 1) / 2 + 1, bnx - 2), J = min((j - 1) / 2 + 1, bny - 2),
                       K = min((k - 1) / 2 + 1, bnz - 2);
-            spa[c] += w * spb[(I * bny + J) * bnz + K];
+            spa[c] += w * spb[split_cell(I, J, K, bnx, bny, bnz)];
         }
     __syncthreads();
     smooth_a(post);
@@ -386,8 +437,9 @@ __device__ __forceinline__ void bottom_core(const BottomSmem& S, BottomCells<KA,
 #pragma unroll
         for (int colour = 0; colour < 2; ++colour)
 #pragma unroll
-            for (int m = 0; m < KB; ++m)
-                if (B[colour][m].d >= 0.0f) st(bb, B[colour][m].c, bvals[colour][m]);  // fluid cells
+            for (int m = 0; m < MB; ++m)
+                if (B[colour][m].d >= 0.0f)  // fluid cells
+                    st(bb, S.list_b[colour * lb + threadIdx.x + m * BOTTOM_THREADS], bvals[colour][m]);
     }
 }
 
@@ -421,8 +473,8 @@ __device__ __forceinline__ void bottom_visit_block(float* __restrict__ pa, const
     const int bsx = bny * bnz, bsy = bnz;
     for (int c = threadIdx.x; c < CA; c += BOTTOM_THREADS) st(pa, c, S.spa[c]);
     for (int c = threadIdx.x; c < CB; c += BOTTOM_THREADS) {
-        st(pb, c, S.spb[c]);
         const int I = c / bsx, J = (c / bsy) % bny, K = c % bnz;
+        st(pb, c, interior(I, J, K, bnx, bny, bnz) ? S.spb[split_cell(I, J, K, bnx, bny, bnz)] : 0.0f);
         // multigrid.cl:115 zeroes b off the interior; cells that are not fluid restrict to 0
         if (!interior(I, J, K, bnx, bny, bnz) || S.sob[c].x < 0.0f) st(bb, c, 0.0f);
     }

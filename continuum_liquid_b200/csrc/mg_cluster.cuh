@@ -100,6 +100,7 @@ __host__ __device__ __forceinline__ long long cluster_lists_slab_ints(const Clus
 struct SlabCell {
     int c;
     float d;
+    float r;  // 1 / d
     float d2b;
 };
 
@@ -179,6 +180,7 @@ __device__ void cluster_slab_path(int s, int cs, const float* __restrict__ pc, f
             SlabCell& o = C[colour][m];
             o.c = c < 0 ? 0 : c;
             o.d = c < 0 ? -1.0f : op4(c).x;
+            o.r = 1.0f / o.d;
             o.d2b = c < 0 ? 0.0f : d2 * sb[c - PL];
         }
 
@@ -209,7 +211,7 @@ __device__ void cluster_slab_path(int s, int cs, const float* __restrict__ pc, f
             const float4 self = op4(c);
             const float ws = self.y * sp[c + PL] + op4(c - PL).y * sp[c - PL] + self.z * sp[c + nz] +
                              op4(c - nz).z * sp[c - nz] + self.w * sp[c + 1] + op4(c - 1).w * sp[c - 1];
-            sp[c] = stored((ws - o.d2b) / o.d);
+            sp[c] = stored(divide_by(ws - o.d2b, o.d, o.r));
         }
         push();
     };
