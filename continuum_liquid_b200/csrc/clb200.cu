@@ -731,7 +731,7 @@ static bool cluster_shape(const clb_mg_hierarchy* h, int level, ClusterShape& ou
     const int* b = h->shape[level + 2];
     const int sa = colour_slots(a[0], a[1], a[2]), sb = colour_slots(b[0], b[1], b[2]);
     const int ka = (sa + BOTTOM_THREADS - 1) / BOTTOM_THREADS, kb = (sb + BOTTOM_BTHREADS - 1) / BOTTOM_BTHREADS;
-    if (kb > 1 || ka > 4) return false;
+    if (bottom_kb(kb) > 1 || ka > 4) return false;  // one cell of B per thread and colour
     const int pairs = (c[0] - 1) / 2;
     const int cs = pairs < CLUSTER_MAX - 1 ? pairs : CLUSTER_MAX - 1;
     if (cs < 1) return false;

@@ -105,12 +105,35 @@ __device__ __forceinline__ float relaxed_w(const OwnedCellW& o, const float* sp,
 }
 
 // One red-black update of an owned cell (multigrid.cl:225-229), p and weights in shared memory.
-__device__ __forceinline__ void relax(const OwnedCell& o, float* sp, const float4* so, int sx, int sy) {
+__device__ __forceinline__ float relaxed(const OwnedCell& o, const float* sp, const float4* so, int sx, int sy) {
     const int c = o.c;
     const float4 self = so[c];
     const float ws = self.y * sp[c + sx] + so[c - sx].y * sp[c - sx] + self.z * sp[c + sy] + so[c - sy].z * sp[c - sy] +
                      self.w * sp[c + 1] + so[c - 1].w * sp[c - 1];
-    sp[c] = divide_by(ws - o.d2b, o.d, o.r);
+    return divide_by(ws - o.d2b, o.d, o.r);
+}
+
+// The updates of a warp's owned slots 0 .. active - 1 of one colour (active is the same in the whole warp), two
+// at a time with both cells' loads ahead of either store: the cells of a colour are independent, and a phase
+// costs what its chains of loads and additions take, one after the other or side by side.
+template <int K, class Value, class Put>
+__device__ __forceinline__ void relax_slots(int active, Value&& value, Put&& put) {
+#pragma unroll
+    for (int m = 0; m < K; m += 2) {
+        if (m + 1 < K && m + 1 < active) {
+            const float a = value(m), b = value(m + 1);
+            put(m, a);
+            put(m + 1, b);
+        } else if (m < active) {
+            put(m, value(m));
+        }
+    }
+}
+
+// Slots in use by this warp when `count` cells go to `threads` threads in turn.
+__device__ __forceinline__ int active_slots(int count, int threads) {
+    const int first = (int)(threadIdx.x & ~31u);
+    return count > first ? (count - first + threads - 1) / threads : 0;
 }
 
 // The coarsest level B: thread t owns the fluid cells t, t + 512 of either colour (bottom_lists), so the first
@@ -264,8 +287,8 @@ __device__ __forceinline__ void bottom_cells(const BottomSmem& S, BottomCells<KA
             const int r = threadIdx.x + m * BOTTOM_THREADS;
             const int c = r < S.count[colour] ? S.list_a[colour * la + r] : -1;
             OwnedCell& o = R.A[colour][m];
-            o.c = c < 0 ? 0 : c;
-            o.d = c < 0 ? -1.0f : S.soa[c].x;  // fluid: >= 0
+            o.c = c < 0 ? (any + 1) * anz + 1 : c;  // a slot without a cell loads an interior cell and stores nothing
+            o.d = c < 0 ? -1.0f : S.soa[c].x;       // fluid: >= 0
             o.r = 1.0f / o.d;
             o.d2b = 0.0f;
         }
@@ -338,13 +361,16 @@ __device__ __forceinline__ void bottom_core(const BottomSmem& S, BottomCells<KA,
     OwnedCell (&A)[2][KA] = R.A;
     OwnedCellW (&B)[2][MB] = R.B;
 
+    const int aslots[2] = {active_slots(S.count[0], BOTTOM_THREADS), active_slots(S.count[1], BOTTOM_THREADS)};
     auto smooth_a = [&](int iterations) {
         for (int it = 0; it < iterations; ++it)
 #pragma unroll
             for (int colour = 0; colour < 2; ++colour) {
-#pragma unroll
-                for (int m = 0; m < KA; ++m)
-                    if (A[colour][m].d > 0.0f) relax(A[colour][m], spa, soa, asx, asy);
+                relax_slots<KA>(
+                    aslots[colour], [&](int m) { return relaxed(A[colour][m], spa, soa, asx, asy); },
+                    [&](int m, float v) {
+                        if (A[colour][m].d > 0.0f) spa[A[colour][m].c] = v;
+                    });
                 __syncthreads();
             }
     };

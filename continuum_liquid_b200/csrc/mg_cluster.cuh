@@ -178,7 +178,7 @@ __device__ void cluster_slab_path(int s, int cs, const float* __restrict__ pc, f
             const int r = threadIdx.x + m * BOTTOM_THREADS;
             const int c = r < counts[colour] ? src[colour * L.list_len + r] : -1;
             SlabCell& o = C[colour][m];
-            o.c = c < 0 ? 0 : c;
+            o.c = c < 0 ? PL + nz + 1 : c;  // a slot without a cell loads an interior cell and stores nothing
             o.d = c < 0 ? -1.0f : op4(c).x;
             o.r = 1.0f / o.d;
             o.d2b = c < 0 ? 0.0f : d2 * sb[c - PL];
@@ -202,17 +202,21 @@ __device__ void cluster_slab_path(int s, int cs, const float* __restrict__ pc, f
             for (int q = threadIdx.x; q < PL; q += BOTTOM_THREADS) right_ghost[q] = sp[own * PL + q];
         cluster_barrier();
     };
+    const int slots[2] = {active_slots(counts[0], BOTTOM_THREADS), active_slots(counts[1], BOTTOM_THREADS)};
     auto phase = [&](int colour) {
-#pragma unroll
-        for (int m = 0; m < NS; ++m) {
-            const SlabCell& o = C[colour][m];
-            if (!(o.d > 0.0f)) continue;
-            const int c = o.c;
-            const float4 self = op4(c);
-            const float ws = self.y * sp[c + PL] + op4(c - PL).y * sp[c - PL] + self.z * sp[c + nz] +
-                             op4(c - nz).z * sp[c - nz] + self.w * sp[c + 1] + op4(c - 1).w * sp[c - 1];
-            sp[c] = stored(divide_by(ws - o.d2b, o.d, o.r));
-        }
+        relax_slots<NS>(
+            slots[colour],
+            [&](int m) {
+                const SlabCell& o = C[colour][m];
+                const int c = o.c;
+                const float4 self = op4(c);
+                const float ws = self.y * sp[c + PL] + op4(c - PL).y * sp[c - PL] + self.z * sp[c + nz] +
+                                 op4(c - nz).z * sp[c - nz] + self.w * sp[c + 1] + op4(c - 1).w * sp[c - 1];
+                return stored(divide_by(ws - o.d2b, o.d, o.r));
+            },
+            [&](int m, float v) {
+                if (C[colour][m].d > 0.0f) sp[C[colour][m].c] = v;
+            });
         push();
     };
 
