@@ -384,20 +384,29 @@ __global__ void __launch_bounds__(COARSE_THREADS) kb_coarse_solve(BList L, const
 }
 
 // ---- FP64 reductions: `R` blocks per scene (block b works for scene b / R) ------------------------------
-template <typename PT_, int MODE>
-__global__ void __launch_bounds__(RN_THREADS) kb_residual_rows(const clb_batch_scene* __restrict__ G, int R,
-                                                               const PT_* p_in, const float* e, double* p_out,
+template <typename PT_>
+__global__ void __launch_bounds__(RN_THREADS) kb_residual_rows(const clb_batch_scene* __restrict__ G, int R, const PT_* p,
                                                                const float* b, const uint8_t* op0, float* r_out,
-                                                               double2* partials, const float* d_in, float* d_out,
-                                                               const double* state) {
+                                                               double2* partials) {
     const int s = blockIdx.x / R, blk = blockIdx.x - s * R;
     const clb_batch_scene& g = G[s];
     const i64 o = g.base[0];
     const double inv_delta2 = 1.0 / ((double)g.delta * (double)g.delta);
-    residual_rows_block<PT_, MODE>(blk, R, p_in + o, e ? e + o : nullptr, p_out ? p_out + o : nullptr, b + o, op0 + o,
-                                   inv_delta2, CLB_DIMS(g, 0), r_out ? r_out + o : nullptr, partials + blockIdx.x,
-                                   d_in ? d_in + o : nullptr, d_out ? d_out + o : nullptr,
-                                   state ? state + 4 * s : nullptr);
+    residual_rows_block<PT_>(blk, R, p + o, b + o, op0 + o, inv_delta2, CLB_DIMS(g, 0), r_out ? r_out + o : nullptr,
+                             partials + blockIdx.x);
+}
+
+// The flexible-CG step's new pressure and direction, `R` blocks per scene (no sums: any R).
+__global__ void __launch_bounds__(RN_THREADS) kb_step_rows(const clb_batch_scene* __restrict__ G, int R,
+                                                           const double* p_in, const float* e, double* p_out,
+                                                           const uint8_t* op0, const float* d_in, float* d_out,
+                                                           const double* state, bool aligned) {
+    const int s = blockIdx.x / R, blk = blockIdx.x - s * R;
+    const clb_batch_scene& g = G[s];
+    const i64 o = g.base[0];
+    const bool vec = aligned && g.shape[0][2] % 4 == 0 && (o & 3) == 0;
+    step_rows_block<RES_FCG, false>(blk, R, p_in + o, e + o, p_out + o, op0 + o, CLB_DIMS(g, 0), d_in + o, d_out + o,
+                                    state + 4 * s, vec);
 }
 
 __global__ void kb_reduce_partials(int R, const double2* partials, double2* out) {

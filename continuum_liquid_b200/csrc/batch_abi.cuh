@@ -264,13 +264,11 @@ int clb_batch_residual_norms(const clb_batch* b, const void* p, int p_is_double,
     cudaStream_t s = CLB_STREAM(stream);
     const int R = b->reduce_blocks;
     if (p_is_double)
-        kb_residual_rows<double, RES_NORM><<<b->scenes * R, RN_THREADS, 0, s>>>(
-            b->geom, R, (const double*)p, nullptr, nullptr, rhs, b->op0, r_out, (double2*)partials, nullptr, nullptr,
-            nullptr);
+        kb_residual_rows<double><<<b->scenes * R, RN_THREADS, 0, s>>>(b->geom, R, (const double*)p, rhs, b->op0, r_out,
+                                                                     (double2*)partials);
     else
-        kb_residual_rows<float, RES_NORM><<<b->scenes * R, RN_THREADS, 0, s>>>(
-            b->geom, R, (const float*)p, nullptr, nullptr, rhs, b->op0, r_out, (double2*)partials, nullptr, nullptr,
-            nullptr);
+        kb_residual_rows<float><<<b->scenes * R, RN_THREADS, 0, s>>>(b->geom, R, (const float*)p, rhs, b->op0, r_out,
+                                                                    (double2*)partials);
     CLB_LAUNCH_CHECK("kb_residual_rows");
     kb_reduce_partials<<<b->scenes, 256, 0, s>>>(R, (const double2*)partials, (double2*)out);
     CLB_LAUNCH_CHECK("kb_reduce_partials");
@@ -317,8 +315,12 @@ int clb_batch_fcg_step(const clb_batch* b, const double* p64_in, const float* z,
     CLB_REQUIRE(p64_in != p64_out && d_in != d_out, "batch_fcg_step: outputs must not alias inputs");
     cudaStream_t s = CLB_STREAM(stream);
     const int R = b->reduce_blocks;
-    kb_residual_rows<double, RES_FCG><<<b->scenes * R, RN_THREADS, 0, s>>>(
-        b->geom, R, p64_in, z, p64_out, rhs, b->op0, r_out, (double2*)partials, d_in, d_out, state);
+    const int wide = 2 * (g_sm_count > 0 ? g_sm_count : 148) * 8 / b->scenes + 1;  // blocks of 8 warps: 16 an SM
+    kb_step_rows<<<b->scenes * wide, RN_THREADS, 0, s>>>(b->geom, wide, p64_in, z, p64_out, b->op0, d_in, d_out, state,
+                                                        step_rows_vec(p64_in, z, p64_out, b->op0, d_in, d_out, 4));
+    CLB_LAUNCH_CHECK("kb_step_rows");
+    kb_residual_rows<double><<<b->scenes * R, RN_THREADS, 0, s>>>(b->geom, R, p64_out, rhs, b->op0, r_out,
+                                                                 (double2*)partials);
     CLB_LAUNCH_CHECK("kb_residual_rows");
     kb_reduce_partials<<<b->scenes, 256, 0, s>>>(R, (const double2*)partials, (double2*)out);
     CLB_LAUNCH_CHECK("kb_reduce_partials");

@@ -1438,6 +1438,40 @@ int row_grid(i64 cells) {
 }  // namespace
 }  // extern "C++"
 
+extern "C++" {
+namespace {
+// One refinement (RES_IR) or flexible-CG (RES_FCG) step: the new pressure and direction, then the residual.
+template <int MODE>
+int solve_step(const double* p64_in, const float* e, double* p64_out, const float* d_in, float* d_out,
+               const double* state, const float* b, const uint8_t* op0, float delta, int nx, int ny, int nz, float* r_out,
+               void* partials, double* out, cudaStream_t s) {
+    const i64 C = (i64)nx * ny * nz;
+    const double inv_delta2 = 1.0 / ((double)delta * (double)delta);
+    const bool vec = step_rows_vec(p64_in, e, p64_out, op0, d_in, d_out, nz);
+    int blocks;
+    if (g_skip_air) {
+        launch(row_grid<k_step_rows<MODE, true>>(C), RN_THREADS, 0, s)(k_step_rows<MODE, true>, p64_in, e, p64_out, op0, nx,
+                                                                      ny, nz, d_in, d_out, state, vec);
+        CLB_LAUNCH_CHECK("k_step_rows");
+        blocks = row_grid<k_residual_rows<double, true>>(C);
+        launch(blocks, RN_THREADS, 0, s)(k_residual_rows<double, true>, (const double*)p64_out, b, op0, inv_delta2, nx, ny,
+                                         nz, r_out, (double2*)partials);
+    } else {
+        launch(row_grid<k_step_rows<MODE, false>>(C), RN_THREADS, 0, s)(k_step_rows<MODE, false>, p64_in, e, p64_out, op0,
+                                                                       nx, ny, nz, d_in, d_out, state, vec);
+        CLB_LAUNCH_CHECK("k_step_rows");
+        blocks = clb_mg_residual_partials(C);
+        launch(blocks, RN_THREADS, 0, s)(k_residual_rows<double, false>, (const double*)p64_out, b, op0, inv_delta2, nx, ny,
+                                         nz, r_out, (double2*)partials);
+    }
+    CLB_LAUNCH_CHECK("k_residual_rows");
+    launch(1, 256, 0, s)(k_reduce_partials, (const double2*)partials, blocks, (double2*)out);
+    CLB_LAUNCH_CHECK("k_reduce_partials");
+    return 0;
+}
+}  // namespace
+}  // extern "C++"
+
 int clb_mg_residual_norms(const void* p, int p_is_double, const float* b, const uint8_t* op0, float delta, int nx,
                           int ny, int nz, float* r_out, void* partials, double* out, void* stream) {
     CLB_GRID_ARGS_OK(nx, ny, nz);
@@ -1447,13 +1481,11 @@ int clb_mg_residual_norms(const void* p, int p_is_double, const float* b, const 
     const double inv_delta2 = 1.0 / ((double)delta * (double)delta);
     cudaStream_t s = CLB_STREAM(stream);
     if (p_is_double)
-        launch(blocks, RN_THREADS, 0, s)(k_residual_rows<double, RES_NORM>, (const double*)p, nullptr, nullptr, b, op0,
-                                         inv_delta2, nx, ny, nz, r_out,
-                                         (double2*)partials, nullptr, nullptr, nullptr);
+        launch(blocks, RN_THREADS, 0, s)(k_residual_rows<double>, (const double*)p, b, op0, inv_delta2, nx, ny, nz, r_out,
+                                         (double2*)partials);
     else
-        launch(blocks, RN_THREADS, 0, s)(k_residual_rows<float, RES_NORM>, (const float*)p, nullptr, nullptr, b, op0,
-                                         inv_delta2, nx, ny, nz, r_out, (double2*)partials,
-                                         nullptr, nullptr, nullptr);
+        launch(blocks, RN_THREADS, 0, s)(k_residual_rows<float>, (const float*)p, b, op0, inv_delta2, nx, ny, nz, r_out,
+                                         (double2*)partials);
     CLB_LAUNCH_CHECK("k_residual_rows");
     launch(1, 256, 0, s)(k_reduce_partials, (const double2*)partials, blocks, (double2*)out);
     CLB_LAUNCH_CHECK("k_reduce_partials");
@@ -1465,23 +1497,8 @@ int clb_mg_ir_step(const double* p64_in, const float* e, double* p64_out, const 
     CLB_GRID_ARGS_OK(nx, ny, nz);
     CLB_REQUIRE(p64_in && e && p64_out && b && op0 && r_out && partials && out, "mg_ir_step: null pointer");
     CLB_REQUIRE(p64_in != p64_out, "mg_ir_step: p64_out must not alias p64_in");
-    const i64 C = (i64)nx * ny * nz;
-    const double inv_delta2 = 1.0 / ((double)delta * (double)delta);
-    cudaStream_t s = CLB_STREAM(stream);
-    int blocks;
-    if (g_skip_air) {
-        blocks = row_grid<k_residual_rows<double, RES_IR, true>>(C);
-        launch(blocks, RN_THREADS, 0, s)(k_residual_rows<double, RES_IR, true>, p64_in, e, p64_out, b, op0, inv_delta2,
-                                         nx, ny, nz, r_out, (double2*)partials, nullptr, nullptr, nullptr);
-    } else {
-        blocks = clb_mg_residual_partials(C);
-        launch(blocks, RN_THREADS, 0, s)(k_residual_rows<double, RES_IR, false>, p64_in, e, p64_out, b, op0,
-                                         inv_delta2, nx, ny, nz, r_out, (double2*)partials, nullptr, nullptr, nullptr);
-    }
-    CLB_LAUNCH_CHECK("k_residual_rows");
-    launch(1, 256, 0, s)(k_reduce_partials, (const double2*)partials, blocks, (double2*)out);
-    CLB_LAUNCH_CHECK("k_reduce_partials");
-    return 0;
+    return solve_step<RES_IR>(p64_in, e, p64_out, nullptr, nullptr, nullptr, b, op0, delta, nx, ny, nz, r_out, partials, out,
+                              CLB_STREAM(stream));
 }
 
 int clb_mg_fcg_dots(const float* z, const float* d, const float* r, const uint8_t* op0, float delta, int nx, int ny,
@@ -1506,23 +1523,8 @@ int clb_mg_fcg_step(const double* p64_in, const float* z, const float* d_in, dou
     CLB_REQUIRE(p64_in && z && d_in && p64_out && d_out && state && b && op0 && r_out && partials && out,
                 "mg_fcg_step: null pointer");
     CLB_REQUIRE(p64_in != p64_out && d_in != d_out, "mg_fcg_step: outputs must not alias inputs");
-    const i64 C = (i64)nx * ny * nz;
-    const double inv_delta2 = 1.0 / ((double)delta * (double)delta);
-    cudaStream_t s = CLB_STREAM(stream);
-    int blocks;
-    if (g_skip_air) {
-        blocks = row_grid<k_residual_rows<double, RES_FCG, true>>(C);
-        launch(blocks, RN_THREADS, 0, s)(k_residual_rows<double, RES_FCG, true>, p64_in, z, p64_out, b, op0,
-                                         inv_delta2, nx, ny, nz, r_out, (double2*)partials, d_in, d_out, state);
-    } else {
-        blocks = clb_mg_residual_partials(C);
-        launch(blocks, RN_THREADS, 0, s)(k_residual_rows<double, RES_FCG, false>, p64_in, z, p64_out, b, op0,
-                                         inv_delta2, nx, ny, nz, r_out, (double2*)partials, d_in, d_out, state);
-    }
-    CLB_LAUNCH_CHECK("k_residual_rows");
-    launch(1, 256, 0, s)(k_reduce_partials, (const double2*)partials, blocks, (double2*)out);
-    CLB_LAUNCH_CHECK("k_reduce_partials");
-    return 0;
+    return solve_step<RES_FCG>(p64_in, z, p64_out, d_in, d_out, state, b, op0, delta, nx, ny, nz, r_out, partials, out,
+                               CLB_STREAM(stream));
 }
 
 int clb_mg_ir_init(const float* p32, const uint8_t* op0, double* p64, int nx, int ny, int nz, void* stream) {

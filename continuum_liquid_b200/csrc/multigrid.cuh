@@ -483,20 +483,24 @@ constexpr int RN_THREADS = 256;
 
 // FP64 residual over the finest level, one (i, j) row per warp (lanes stride along k, so there is no
 // per-cell index division). Per block: sums of r^2 and b^2 over interior fluid cells, with
-// r = b - A p evaluated in FP64 (A is multigrid.cl:25-43 apply_operator).
-//  MODE 0 (RES_NORM): p is the float or double pressure p_in.
-//  MODE 1 (RES_IR):   the refinement update fused in: p = p_in + e is formed on the fly for the cell
-//                     and its neighbours and written to p_out (which must not alias p_in).
-//  MODE 2 (RES_FCG):  the flexible-CG update fused in: the search direction d = e + beta d_in
-//                     (rounded to float, written to d_out) and p = p_in + alpha d, with alpha and
-//                     beta read from state[0] and state[1] (k_fcg_scalars).
+// r = b - A p evaluated in FP64 (A is multigrid.cl:25-43 apply_operator) of the float or double pressure p.
 // When r_out is given the residual is stored rounded to float at every cell (0 outside interior
 // fluid cells): it is the right-hand side of the next correction solve.
+//
+// The refinement and flexible-CG steps first form the new pressure cell by cell (step_rows_block), then
+// take its residual here:
+//  RES_IR:   p_out = p_in + e
+//  RES_FCG:  the search direction d = e + beta d_in (rounded to float, written to d_out) and
+//            p_out = p_in + alpha d, with alpha and beta read from state[0] and state[1] (k_fcg_scalars).
+// One pass that forms the neighbours' new pressures as it needs them reads less, but converts between float and
+// double about 34 times a cell, at an eighth of the rate of the additions. A step's launches (B200, us, cold
+// cache): six scenes of 48^3-96^3 14 + 65 (184 in one pass), 128^3 pool 27 in one pass, 256^3 block 25 + 39 (63).
+// Bound by the latency of a row's rounds of loads (two cells of a lane at a time) at 24-32 warps an SM.
 // SKIP (refinement and FCG steps): cells that are not interior fluid cells are neither read nor
 // written. Every value there is 0 when the caller keeps the invariant (e, d_in, p_in, and the
 // outputs zeroed outside the fluid once per solve), so the outputs and sums are those of the full
 // pass; the per-lane summation order over fluid cells is unchanged.
-enum { RES_NORM = 0, RES_IR = 1, RES_FCG = 2 };
+enum { RES_IR = 1, RES_FCG = 2 };
 
 // Whether row `base` (nz cells of the packed finest operator) holds a fluid cell, for the whole warp:
 // one 8-byte load per lane per 256 cells (when the row starts 8-byte aligned) instead of the per-cell
@@ -520,69 +524,175 @@ __device__ __forceinline__ bool row_has_fluid(const uint8_t* __restrict__ op0, i
     return __any_sync(0xffffffffu, any);
 }
 
-// Block `blk` of `nblk` blocks sharing the rows; its partial sums go to *partial.
-template <typename PT, int MODE, bool SKIP = false>
-__device__ __forceinline__ void residual_rows_block(int blk, int nblk, const PT* __restrict__ p_in,
-                                                    const float* __restrict__ e, double* __restrict__ p_out,
-                                                    const float* __restrict__ b, const uint8_t* __restrict__ op0,
-                                                    double inv_delta2, int nx, int ny, int nz,
-                                                    float* __restrict__ r_out, double2* __restrict__ partial,
-                                                    const float* __restrict__ d_in, float* __restrict__ d_out,
-                                                    const double* __restrict__ state) {
-    __shared__ double2 s_red[RN_THREADS / 32];
+// The new pressure (and direction) of the rows of block `blk` of `nblk`, a warp per row. vec: nz is a multiple of 4 and
+// every array 16-byte aligned (op0 4-byte), so a lane takes four cells with 16-byte loads and stores.
+template <int MODE, bool SKIP>
+__device__ __forceinline__ void step_rows_block(int blk, int nblk, const double* __restrict__ p_in,
+                                                const float* __restrict__ e, double* __restrict__ p_out,
+                                                const uint8_t* __restrict__ op0, int nx, int ny, int nz,
+                                                const float* __restrict__ d_in, float* __restrict__ d_out,
+                                                const double* __restrict__ state, bool vec) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int sx = ny * nz, sy = nz;
-    double rr = 0.0, bb = 0.0;
     double alpha = 0.0, beta = 0.0;
     if (MODE == RES_FCG) {
         alpha = state[0];
         beta = state[1];
     }
-    auto dv = [&](int q) -> float { return (float)((double)__ldg(e + q) + beta * (double)__ldg(d_in + q)); };
-    auto pv = [&](int q) -> double {
-        if (MODE == RES_IR) return (double)__ldg(p_in + q) + (double)__ldg(e + q);
-        if (MODE == RES_FCG) return (double)__ldg(p_in + q) + alpha * (double)dv(q);
-        return (double)__ldg(p_in + q);
-    };
+    auto direction = [&](float ev, float dv) { return (float)((double)ev + beta * (double)dv); };
+    const int rows = nx * ny;
+    for (int r = blk * (RN_THREADS / 32) + warp; r < rows; r += nblk * (RN_THREADS / 32)) {
+        const int i = r / ny, j = r - i * ny;
+        const int base = r * nz;
+        if (SKIP && (i < 1 || i > nx - 2 || j < 1 || j > ny - 2 || !row_has_fluid(op0, base, nz, lane))) continue;
+        if (vec) {
+#pragma unroll 2
+            for (int k = 4 * lane; k < nz; k += 128) {
+                const int c = base + k;
+                bool in[4] = {true, true, true, true};
+                if (SKIP) {
+                    const uchar4 o = __ldg(reinterpret_cast<const uchar4*>(op0 + c));
+                    in[0] = (o.x & 64u) && k >= 1;
+                    in[1] = (o.y & 64u) != 0u;
+                    in[2] = (o.z & 64u) != 0u;
+                    in[3] = (o.w & 64u) && k + 3 <= nz - 2;
+                    if (!(in[0] || in[1] || in[2] || in[3])) continue;
+                }
+                const float4 ev = __ldg(reinterpret_cast<const float4*>(e + c));
+                const double2 pa = __ldg(reinterpret_cast<const double2*>(p_in + c));
+                const double2 pb = __ldg(reinterpret_cast<const double2*>(p_in + c) + 1);
+                float4 dv = ev;
+                if (MODE == RES_FCG) {
+                    const float4 di = __ldg(reinterpret_cast<const float4*>(d_in + c));
+                    dv = make_float4(direction(ev.x, di.x), direction(ev.y, di.y), direction(ev.z, di.z),
+                                     direction(ev.w, di.w));
+                }
+                const float dn[4] = {dv.x, dv.y, dv.z, dv.w};
+                const double pi[4] = {pa.x, pa.y, pb.x, pb.y};
+                double pn[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) pn[q] = pi[q] + (MODE == RES_FCG ? alpha * (double)dn[q] : (double)dn[q]);
+                if (in[0] && in[1] && in[2] && in[3]) {
+                    reinterpret_cast<double2*>(p_out + c)[0] = make_double2(pn[0], pn[1]);
+                    reinterpret_cast<double2*>(p_out + c)[1] = make_double2(pn[2], pn[3]);
+                    if (MODE == RES_FCG) *reinterpret_cast<float4*>(d_out + c) = dv;
+                } else {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        if (in[q]) {
+                            p_out[c + q] = pn[q];
+                            if (MODE == RES_FCG) d_out[c + q] = dn[q];
+                        }
+                }
+            }
+        } else {
+#pragma unroll 2
+            for (int k = lane; k < nz; k += 32) {
+                const int c = base + k;
+                if (SKIP && !(k >= 1 && k <= nz - 2 && (__ldg(op0 + c) & 64u))) continue;
+                const float ev = __ldg(e + c);
+                const float dv = MODE == RES_FCG ? direction(ev, __ldg(d_in + c)) : ev;
+                p_out[c] = __ldg(p_in + c) + (MODE == RES_FCG ? alpha * (double)dv : (double)dv);
+                if (MODE == RES_FCG) d_out[c] = dv;
+            }
+        }
+    }
+}
+
+template <int MODE, bool SKIP>
+__global__ void __launch_bounds__(RN_THREADS) k_step_rows(const double* __restrict__ p_in, const float* __restrict__ e,
+                                                           double* __restrict__ p_out,
+                                                           const uint8_t* __restrict__ op0, int nx, int ny, int nz,
+                                                           const float* __restrict__ d_in, float* __restrict__ d_out,
+                                                           const double* __restrict__ state, bool vec) {
+    pdl_begin();
+    step_rows_block<MODE, SKIP>(blockIdx.x, gridDim.x, p_in, e, p_out, op0, nx, ny, nz, d_in, d_out, state, vec);
+}
+
+// Whether step_rows_block may take four cells at a time.
+static inline bool step_rows_vec(const void* p_in, const void* e, const void* p_out, const void* op0, const void* d_in,
+                                 const void* d_out, int nz) {
+    return nz % 4 == 0 && (((uintptr_t)op0) & 3) == 0 &&
+           (((uintptr_t)p_in | (uintptr_t)e | (uintptr_t)p_out | (uintptr_t)d_in | (uintptr_t)d_out) & 15) == 0;
+}
+
+// The finest level's neighbour sum in FP64, in the reference's order, from the six neighbours' values (x + 1, x - 1,
+// y + 1, ...) and the operator bytes of the cell and its three lower neighbours: each weight is 0 or 1.
+template <typename T>
+__device__ __forceinline__ double weighted(uint32_t o, uint32_t ox, uint32_t oy, uint32_t oz, const T* nb) {
+    auto w = [](uint32_t bit, T v) { return bit ? (double)v : 0.0; };
+    return w(o & 8u, nb[0]) + w(ox & 8u, nb[1]) + w(o & 16u, nb[2]) + w(oy & 16u, nb[3]) + w(o & 32u, nb[4]) +
+           w(oz & 32u, nb[5]);
+}
+
+// Block `blk` of `nblk` blocks sharing the rows; its partial sums go to *partial.
+template <typename PT, bool SKIP = false>
+__device__ __forceinline__ void residual_rows_block(int blk, int nblk, const PT* p, const float* __restrict__ b,
+                                                    const uint8_t* __restrict__ op0, double inv_delta2, int nx, int ny,
+                                                    int nz, float* __restrict__ r_out, double2* __restrict__ partial) {
+    __shared__ double2 s_red[RN_THREADS / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int sx = ny * nz, sy = nz;
+    double rr = 0.0, bb = 0.0;
     const int rows = nx * ny;
     for (int r = blk * (RN_THREADS / 32) + warp; r < rows; r += nblk * (RN_THREADS / 32)) {
         const int i = r / ny, j = r - i * ny;
         const bool row_in = i >= 1 && i <= nx - 2 && j >= 1 && j <= ny - 2;
         const int base = r * nz;
-        if (SKIP && MODE != RES_NORM && (!row_in || !row_has_fluid(op0, base, nz, lane))) continue;
-        // a lane's operator bytes of 8 consecutive steps are loaded together, so a step waits on one
-        // round of loads (its stencil), not two (the byte that says whether the cell is fluid first)
+        if (!row_in || !row_has_fluid(op0, base, nz, lane)) {
+            if (!SKIP && r_out)
+                for (int k = lane; k < nz; k += 32) r_out[base + k] = 0.0f;
+            continue;
+        }
+        // a lane's operator bytes of 8 consecutive steps are loaded together, and its cells are taken two at a
+        // time, both stencils' loads ahead of either sum: a row is a chain of four rounds of loads per 256 cells
         for (int k0 = 0; k0 < nz; k0 += 256) {
-        unsigned long long ops = 0ull;  // byte m: the operator of step m
+            unsigned long long ops = 0ull;  // byte m: the operator of step m
 #pragma unroll
-        for (int m = 0; m < 8; ++m) {
-            const int k = k0 + lane + 32 * m;
-            if (k < nz) ops |= (unsigned long long)__ldg(op0 + base + k) << (8 * m);
-        }
-#pragma unroll 1
-        for (int m = 0; m < 8; ++m) {
-            const int k = k0 + lane + 32 * m;
-            if (k >= nz) continue;
-            const int c = base + k;
-            const uint32_t o = (uint32_t)(ops >> (8 * m)) & 0xffu;
-            if (SKIP && MODE != RES_NORM && !(row_in && k >= 1 && k <= nz - 2 && (o & 64u))) continue;
-            const double pc = pv(c);
-            if (MODE != RES_NORM) p_out[c] = pc;
-            if (MODE == RES_FCG) d_out[c] = dv(c);
-            float rf = 0.0f;
-            if (row_in && k >= 1 && k <= nz - 2 && (o & 64u)) {
-                const uint32_t ox = __ldg(op0 + c - sx), oy = __ldg(op0 + c - sy), oz = __ldg(op0 + c - 1);
-                const double ws = (double)bitf(o, 3) * pv(c + sx) + (double)bitf(ox, 3) * pv(c - sx) +
-                                  (double)bitf(o, 4) * pv(c + sy) + (double)bitf(oy, 4) * pv(c - sy) +
-                                  (double)bitf(o, 5) * pv(c + 1) + (double)bitf(oz, 5) * pv(c - 1);
-                const double bv = (double)__ldg(b + c);
-                const double res = bv - (ws - (double)(o & 7u) * pc) * inv_delta2;
-                rr += res * res;
-                bb += bv * bv;
-                rf = (float)res;
+            for (int m = 0; m < 8; ++m) {
+                const int k = k0 + lane + 32 * m;
+                if (k < nz) ops |= (unsigned long long)__ldg(op0 + base + k) << (8 * m);
             }
-            if (r_out) r_out[c] = rf;
-        }
+#pragma unroll 1
+            for (int m = 0; m < 8; m += 2) {
+                if (k0 + 32 * m >= nz) break;
+                PT pc[2], nb[2][6];
+                float bv[2];
+                uint32_t o[2], ox[2], oy[2], oz[2];
+                bool in[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int k = k0 + lane + 32 * (m + h), c = base + k;
+                    o[h] = (uint32_t)(ops >> (8 * (m + h))) & 0xffu;
+                    in[h] = k >= 1 && k <= nz - 2 && (o[h] & 64u);
+                    if (in[h]) {
+                        ox[h] = __ldg(op0 + c - sx);
+                        oy[h] = __ldg(op0 + c - sy);
+                        oz[h] = __ldg(op0 + c - 1);
+                        pc[h] = p[c];
+                        bv[h] = __ldg(b + c);
+                        nb[h][0] = p[c + sx];
+                        nb[h][1] = p[c - sx];
+                        nb[h][2] = p[c + sy];
+                        nb[h][3] = p[c - sy];
+                        nb[h][4] = p[c + 1];
+                        nb[h][5] = p[c - 1];
+                    }
+                }
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int k = k0 + lane + 32 * (m + h);
+                    float rf = 0.0f;
+                    if (in[h]) {
+                        const double ws = weighted(o[h], ox[h], oy[h], oz[h], nb[h]);
+                        const double bd = (double)bv[h];
+                        const double res = bd - (ws - (double)(o[h] & 7u) * (double)pc[h]) * inv_delta2;
+                        rr += res * res;
+                        bb += bd * bd;
+                        rf = (float)res;
+                    }
+                    if (r_out && (in[h] || (!SKIP && k < nz))) r_out[base + k] = rf;
+                }
+            }
         }
     }
 #pragma unroll
@@ -602,20 +712,13 @@ __device__ __forceinline__ void residual_rows_block(int blk, int nblk, const PT*
     }
 }
 
-template <typename PT, int MODE, bool SKIP = false>
-__global__ void __launch_bounds__(RN_THREADS) k_residual_rows(const PT* __restrict__ p_in,
-                                                               const float* __restrict__ e,
-                                                               double* __restrict__ p_out,
-                                                               const float* __restrict__ b,
+template <typename PT, bool SKIP = false>
+__global__ void __launch_bounds__(RN_THREADS) k_residual_rows(const PT* p, const float* __restrict__ b,
                                                                const uint8_t* __restrict__ op0, double inv_delta2,
                                                                int nx, int ny, int nz, float* __restrict__ r_out,
-                                                               double2* __restrict__ partials,
-                                                               const float* __restrict__ d_in = nullptr,
-                                                               float* __restrict__ d_out = nullptr,
-                                                               const double* __restrict__ state = nullptr) {
+                                                               double2* __restrict__ partials) {
     pdl_begin();
-    residual_rows_block<PT, MODE, SKIP>(blockIdx.x, gridDim.x, p_in, e, p_out, b, op0, inv_delta2, nx, ny, nz, r_out,
-                                  partials + blockIdx.x, d_in, d_out, state);
+    residual_rows_block<PT, SKIP>(blockIdx.x, gridDim.x, p, b, op0, inv_delta2, nx, ny, nz, r_out, partials + blockIdx.x);
 }
 
 // Flexible conjugate gradients with the W-cycle as preconditioner (Notay's FCG with truncation 1;
@@ -644,24 +747,52 @@ __device__ __forceinline__ void fcg_dots_block(int blk, int nblk, const float* _
         if (i < 1 || i > nx - 2 || j < 1 || j > ny - 2) continue;
         const int base = q * nz;
         if (!row_has_fluid(op0, base, nz, lane)) continue;
-        for (int k = lane; k < nz; k += 32) {
-            const int c = base + k;
-            const uint32_t o = __ldg(op0 + c);
-            if (k < 1 || k > nz - 2 || !(o & 64u)) continue;
-            const uint32_t ox = __ldg(op0 + c - sx), oy = __ldg(op0 + c - sy), oz = __ldg(op0 + c - 1);
-            const double zc = (double)__ldg(z + c);
-            const double ws = (double)bitf(o, 3) * (double)__ldg(z + c + sx) +
-                              (double)bitf(ox, 3) * (double)__ldg(z + c - sx) +
-                              (double)bitf(o, 4) * (double)__ldg(z + c + sy) +
-                              (double)bitf(oy, 4) * (double)__ldg(z + c - sy) +
-                              (double)bitf(o, 5) * (double)__ldg(z + c + 1) +
-                              (double)bitf(oz, 5) * (double)__ldg(z + c - 1);
-            const double az = (ws - (double)(o & 7u) * zc) * inv_delta2;
-            const double dc = (double)__ldg(d + c), rc = (double)__ldg(r + c);
-            t.x += az * dc;
-            t.y += az * zc;
-            t.z += zc * rc;
-            t.w += dc * rc;
+        // as residual_rows_block: the operator bytes of eight steps first, then two cells at a time
+        for (int k0 = 0; k0 < nz; k0 += 256) {
+            unsigned long long ops = 0ull;
+#pragma unroll
+            for (int m = 0; m < 8; ++m) {
+                const int k = k0 + lane + 32 * m;
+                if (k < nz) ops |= (unsigned long long)__ldg(op0 + base + k) << (8 * m);
+            }
+#pragma unroll 1
+            for (int m = 0; m < 8; m += 2) {
+                if (k0 + 32 * m >= nz) break;
+                float zc[2], dc[2], rc[2], nb[2][6];
+                uint32_t o[2], ox[2], oy[2], oz[2];
+                bool in[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int k = k0 + lane + 32 * (m + h), c = base + k;
+                    o[h] = (uint32_t)(ops >> (8 * (m + h))) & 0xffu;
+                    in[h] = k >= 1 && k <= nz - 2 && (o[h] & 64u);
+                    if (in[h]) {
+                        ox[h] = __ldg(op0 + c - sx);
+                        oy[h] = __ldg(op0 + c - sy);
+                        oz[h] = __ldg(op0 + c - 1);
+                        zc[h] = __ldg(z + c);
+                        dc[h] = __ldg(d + c);
+                        rc[h] = __ldg(r + c);
+                        nb[h][0] = __ldg(z + c + sx);
+                        nb[h][1] = __ldg(z + c - sx);
+                        nb[h][2] = __ldg(z + c + sy);
+                        nb[h][3] = __ldg(z + c - sy);
+                        nb[h][4] = __ldg(z + c + 1);
+                        nb[h][5] = __ldg(z + c - 1);
+                    }
+                }
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    if (in[h]) {
+                        const double ws = weighted(o[h], ox[h], oy[h], oz[h], nb[h]);
+                        const double zd = (double)zc[h], dd = (double)dc[h], rd = (double)rc[h];
+                        const double az = (ws - (double)(o[h] & 7u) * zd) * inv_delta2;
+                        t.x += az * dd;
+                        t.y += az * zd;
+                        t.z += zd * rd;
+                        t.w += dd * rd;
+                    }
+            }
         }
     }
 #pragma unroll
