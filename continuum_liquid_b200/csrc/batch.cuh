@@ -118,9 +118,61 @@ __global__ void __launch_bounds__(P2G_THREADS) kb_p2g(BList L, i64 total, const 
              w + o, ff + o, g.inv_dx, inv_ppc, CLB_DIMS(g, 0));
 }
 
-// k_p2g_tiled over the batch: the scenes' tiles are numbered scene after scene (in list order), block b
-// runs tile b of that numbering on its scene; bin offsets are batch-wide particle indices.
-__global__ void __launch_bounds__(P2GT_THREADS, 2) kb_p2g_tiled(BList L, const clb_batch_scene* __restrict__ G,
+__host__ __device__ __forceinline__ i64 scene_cells(const clb_batch_scene& g) {
+    return (i64)g.shape[0][0] * g.shape[0][1] * g.shape[0][2];
+}
+
+// start[q + 1] holds the blocks of list entry q; turns them into prefix sums and returns the entry of block b, or -1
+// past the last (the same in the whole block).
+__device__ __forceinline__ int scene_of_block(i64* start, int count, i64 b) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        start[0] = 0;
+        for (int q = 1; q <= count; ++q) start[q] += start[q - 1];
+    }
+    __syncthreads();
+    if (b >= start[count]) return -1;
+    int lo = 0, hi = count - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (start[mid] <= b) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
+// k_p2g_ordered over the batch, likewise: the scenes with fewer than `below` cells.
+__host__ __device__ __forceinline__ i64 p2g_ordered_blocks(int nx, int ny, int nz, int TI) {
+    return p2g_ordered_tiles<0>(nx, ny, nz, TI) + p2g_ordered_tiles<1>(nx, ny, nz, TI) + p2g_ordered_tiles<2>(nx, ny, nz, TI);
+}
+__global__ void __launch_bounds__(P2GO_THREADS, 2) kb_p2g_ordered(BList L, const clb_batch_scene* __restrict__ G,
+                                                                   const float* __restrict__ pos,
+                                                                   const float* __restrict__ vel,
+                                                                   const int* __restrict__ offsets,
+                                                                   const int* __restrict__ counts, float* __restrict__ u,
+                                                                   float* __restrict__ v, float* __restrict__ w,
+                                                                   float* __restrict__ ff, float inv_ppc, i64 below,
+                                                                   float one) {
+    extern __shared__ __align__(16) float p2go_smem[];
+    __shared__ i64 s_start[CLB_BATCH_MAX_SCENES + 1];
+    for (int q = threadIdx.x; q < L.count; q += P2GO_THREADS) {
+        const clb_batch_scene& g = G[L.scene[q]];
+        const i64 C = scene_cells(g);
+        s_start[q + 1] = C >= below ? 0 : p2g_ordered_blocks(CLB_DIMS(g, 0), p2g_ordered_planes(C));
+    }
+    const i64 b = blockIdx.x;
+    const int lo = scene_of_block(s_start, L.count, b);
+    if (lo < 0) return;  // the whole block leaves together
+    const clb_batch_scene& g = G[L.scene[lo]];
+    const i64 o = g.base[0];
+    const P2GGrid grid{g.shape[0][0], g.shape[0][1], g.shape[0][2], p2g_ordered_planes(scene_cells(g)), g.inv_dx, inv_ppc,
+                       one};
+    p2g_ordered_block(p2go_smem, b - s_start[lo], grid, pos, vel, offsets + o, counts + o, u + o, v + o, w + o, ff + o);
+}
+
+// k_p2g_tiled over the batch: the tiles of the scenes of at least P2GT_MIN_CELLS cells are numbered scene after scene
+// (in list order), block b runs tile b of that numbering on its scene; bin offsets are batch-wide particle indices.
+__global__ void __launch_bounds__(P2GT_THREADS, 1) kb_p2g_tiled(BList L, const clb_batch_scene* __restrict__ G,
                                                                  const float* __restrict__ pos,
                                                                  const float* __restrict__ vel,
                                                                  const int* __restrict__ offsets,
@@ -131,22 +183,11 @@ __global__ void __launch_bounds__(P2GT_THREADS, 2) kb_p2g_tiled(BList L, const c
     for (int q = threadIdx.x; q < L.count; q += P2GT_THREADS) {
         const clb_batch_scene& g = G[L.scene[q]];
         int tj, tk;
-        s_start[q + 1] = p2g_tiled_tiles(CLB_DIMS(g, 0), &tj, &tk);
+        s_start[q + 1] = scene_cells(g) < P2GT_MIN_CELLS ? 0 : p2g_tiled_tiles(CLB_DIMS(g, 0), &tj, &tk);
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        s_start[0] = 0;
-        for (int q = 1; q <= L.count; ++q) s_start[q] += s_start[q - 1];
-    }
-    __syncthreads();
     const i64 b = blockIdx.x;
-    if (b >= s_start[L.count]) return;  // the whole block leaves together
-    int lo = 0, hi = L.count - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (s_start[mid] <= b) lo = mid;
-        else hi = mid - 1;
-    }
+    const int lo = scene_of_block(s_start, L.count, b);
+    if (lo < 0) return;  // the whole block leaves together
     const clb_batch_scene& g = G[L.scene[lo]];
     const i64 o = g.base[0];
     int tj, tk;

@@ -163,17 +163,30 @@ int clb_batch_particle_to_grid(const clb_batch* b, const float* particles, const
     if (clb_sort_particles(particles, velocity, particles_work, velocity_work, bin_offsets, bin_counts, keys, ranks,
                            perm, slot_keys, n, stream))
         return 1;
-    if (b->p2g_tiled) {  // each particle visited once per tile (the tolerance mode's P2G)
-        i64 tiles = 0;
+    // the kernels of the single-scene P2G: the ordered walk (tolerance mode: of the scenes below P2GT_MIN_CELLS), the
+    // tiled scatter of larger scenes; the eight-lane gather in the reference mode when all scenes together are small
+    if (b->p2g_tiled || C >= P2GO_MIN_CELLS) {
+        const i64 below = b->p2g_tiled ? P2GT_MIN_CELLS : ((i64)1 << 62);
+        i64 walks = 0, tiles = 0;
         for (int q = 0; q < b->scenes; ++q) {
-            const clb_batch_scene& g = b->geom_host[q];
+            const int* n = b->geom_host[q].shape[0];
+            const i64 cells = scene_cells(b->geom_host[q]);
             int tj, tk;
-            tiles += p2g_tiled_tiles(g.shape[0][0], g.shape[0][1], g.shape[0][2], &tj, &tk);
+            if (cells < below) walks += p2g_ordered_blocks(n[0], n[1], n[2], p2g_ordered_planes(cells));
+            else tiles += p2g_tiled_tiles(n[0], n[1], n[2], &tj, &tk);
         }
-        kb_p2g_tiled<<<(unsigned)tiles, P2GT_THREADS, P2GT_SMEM, s>>>(blist(b->cells[0]), b->geom, particles_work,
-                                                                      velocity_work, bin_offsets, bin_counts, u, v, w,
-                                                                      fluid_fraction, inv_ppc);
-        CLB_LAUNCH_CHECK("kb_p2g_tiled");
+        if (walks > 0) {
+            kb_p2g_ordered<<<(unsigned)walks, P2GO_THREADS, P2GO_SMEM, s>>>(
+                blist(b->cells[0]), b->geom, particles_work, velocity_work, bin_offsets, bin_counts, u, v, w,
+                fluid_fraction, inv_ppc, below, 1.0f);
+            CLB_LAUNCH_CHECK("kb_p2g_ordered");
+        }
+        if (tiles > 0) {
+            kb_p2g_tiled<<<(unsigned)tiles, P2GT_THREADS, P2GT_SMEM, s>>>(blist(b->cells[0]), b->geom, particles_work,
+                                                                          velocity_work, bin_offsets, bin_counts, u, v,
+                                                                          w, fluid_fraction, inv_ppc);
+            CLB_LAUNCH_CHECK("kb_p2g_tiled");
+        }
         return 0;
     }
     kb_p2g<<<blocks_for(C * P2G_LANES, P2G_THREADS), P2G_THREADS, 0, s>>>(

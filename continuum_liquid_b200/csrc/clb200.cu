@@ -160,6 +160,8 @@ int clb_init(int device) {
                    "ordered P2G attribute") ||
         check_call(cudaFuncSetAttribute(k_p2g_tiled, cudaFuncAttributeMaxDynamicSharedMemorySize, P2GT_SMEM),
                    "tiled P2G attribute") ||
+        check_call(cudaFuncSetAttribute(kb_p2g_ordered, cudaFuncAttributeMaxDynamicSharedMemorySize, P2GO_SMEM),
+                   "batched ordered P2G attribute") ||
         check_call(cudaFuncSetAttribute(kb_p2g_tiled, cudaFuncAttributeMaxDynamicSharedMemorySize, P2GT_SMEM),
                    "batched tiled P2G attribute") ||
         check_call(cudaFuncSetAttribute(k_particle_update_tiled<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -281,7 +283,7 @@ int clb_sort_particles(const float* particles, const float* velocity, float* par
 
 // The reference-order P2G: the tile walk of p2g_ordered.cuh, or the gather with eight lanes per cell on grids so small
 // that a tile's chain of planes is longer than the whole gather (28,800 cells: 15 against 29 us; 64^3 with 185,000
-// particles: 48 against 34).
+// particles: 48 against 33).
 static int p2g_reference(const float* particles, const float* velocity, const int32_t* offsets, const int32_t* counts,
                          float* u, float* v, float* w, float* ff, float inv_dx, float inv_ppc, int nx, int ny, int nz,
                          cudaStream_t s) {
@@ -316,6 +318,9 @@ int clb_particle_to_grid_gather_tiled(const float* particles, const float* veloc
     CLB_GRID_ARGS_OK(nx, ny, nz);
     CLB_REQUIRE(bin_offsets && bin_counts && u && v && w && fluid_fraction,
                 "particle_to_grid_gather_tiled: null pointer");
+    if ((i64)nx * ny * nz < P2GT_MIN_CELLS)
+        return p2g_reference(particles, velocity, bin_offsets, bin_counts, u, v, w, fluid_fraction, inv_dx,
+                             inv_particles_per_cell, nx, ny, nz, CLB_STREAM(stream));
     int tiles_j = 0, tiles_k = 0;
     const int tiles = p2g_tiled_tiles(nx, ny, nz, &tiles_j, &tiles_k);
     k_p2g_tiled<<<tiles, P2GT_THREADS, P2GT_SMEM, CLB_STREAM(stream)>>>(particles, velocity, bin_offsets, bin_counts,

@@ -22,9 +22,9 @@
 // the 12 sums of a bin stay in registers at 16 warps an SM, a tile's halo is one-sided along the other axes, and
 // small grids still have enough blocks.
 //
-// Measured (B200, us, against the gather of binning.cuh): 64^3 dam break 34 (48), 117 x 90 x 139 with 4.0M particles 206
-// (539), 160^3 with 5.5M 309 (938), 256^3 with 23M 1185 (3700). 195M instructions at 160^3, 58 % of the issue slots;
-// lanes wait for the fullest bin of a row (about 14 particles against 8 on average).
+// Measured (B200, us, against the gather of binning.cuh): 64^3 dam break 33 (48), 117 x 90 x 139 with 4.0M particles 199
+// (539), 160^3 with 5.5M 297 (938), 256^3 with 23M 1114 (3700). 58 % of the issue slots; lanes wait for the fullest
+// bin of a row (about 14 particles against 8 on average).
 #pragma once
 #include <type_traits>
 #include <utility>
@@ -53,6 +53,17 @@ __device__ __forceinline__ float hi2(f32x2 v) {
 __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
     f32x2 r;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// a + b; the assembler may join it to the paired multiplication that gave b and then rounds once.
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
 // a + b as b * 1 + a, with the 1 from the launch's arguments: the assembler joins a paired addition (or one with a
@@ -145,10 +156,11 @@ struct P2GTile {
     static constexpr int TJ = P2GO_WARPS - (A == 1 ? 2 : 1), TK = 32 - (A == 2 ? 2 : 1), PLANE = TJ * TK;
 };
 constexpr int P2GO_PLANE = 7 * 31;  // cells of the largest plane
-// four planes of eight lanes' velocity and weight sums, four planes of counts, the warps' buffers
+// four planes of eight lanes' velocity and weight sums (and two planes' space for one sum that no cell has), four
+// planes of counts, the warps' buffers
 constexpr int P2GO_BUFFER = P2GO_ROW * 4 + 4;  // positions from a 16-byte boundary on, then the velocity component
-constexpr int P2GO_SMEM = (4 * 16 * P2GO_PLANE + 4 * P2GO_PLANE + P2GO_WARPS * P2GO_BUFFER) * 4;
-static_assert((P2GO_ROW * 3 + 4) % 4 == 0 && P2GO_BUFFER % 4 == 0 && (68 * P2GO_PLANE) % 4 == 0, "16-byte buffers");
+constexpr int P2GO_SMEM = (70 * P2GO_PLANE + P2GO_WARPS * P2GO_BUFFER + 2) * 4;
+static_assert((P2GO_ROW * 3 + 4) % 4 == 0 && P2GO_BUFFER % 4 == 0 && (70 * P2GO_PLANE + 2) % 4 == 0, "16-byte buffers");
 
 struct P2GGrid {
     int nx, ny, nz, TI;
@@ -164,9 +176,9 @@ __device__ __forceinline__ void p2g_ordered_tile(float* smem, int tile, const P2
     constexpr int TJ = P2GTile<A>::TJ, TK = P2GTile<A>::TK, PLANE = P2GTile<A>::PLANE;
     const int nx = g.nx, ny = g.ny, nz = g.nz, TI = g.TI;
     float* sums = smem;  // [ring slot][lane][velocity, weight][cell of the plane]
-    int* count = reinterpret_cast<int*>(smem + 64 * P2GO_PLANE);
+    int* count = reinterpret_cast<int*>(smem + 66 * P2GO_PLANE);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float* bp = smem + 68 * P2GO_PLANE + warp * P2GO_BUFFER;
+    float* bp = smem + 70 * P2GO_PLANE + 2 + warp * P2GO_BUFFER;
     float* bv = bp + 3 * P2GO_ROW + 4;
     const uint32_t bp32 = (uint32_t)__cvta_generic_to_shared(bp), bv32 = (uint32_t)__cvta_generic_to_shared(bv);
     const bool aligned = (((uintptr_t)pos) & 15) == 0;
@@ -193,7 +205,7 @@ __device__ __forceinline__ void p2g_ordered_tile(float* smem, int tile, const P2
     }
     any = __syncthreads_or(any);
     if (any) {
-        for (int c = threadIdx.x; c < 68 * P2GO_PLANE / 4; c += P2GO_THREADS)
+        for (int c = threadIdx.x; c < (70 * P2GO_PLANE + 2) / 4; c += P2GO_THREADS)
             reinterpret_cast<float4*>(smem)[c] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         __syncthreads();
     }
@@ -250,13 +262,16 @@ __device__ __forceinline__ void p2g_ordered_tile(float* smem, int tile, const P2
             look_up(li + 1, next_begin, next_n);
             if (first < last) {  // warp-uniform
                 const float fbx = (float)bx, fby = (float)by, fbz = (float)bz;
-                // the place of a role's sums: its lane's of cell b - o, when the tile has that cell
+                // The place of a role's sums: its lane's of cell b - o, or the spare one when the tile does not have that
+                // cell. A lane without particles puts back what it took (0 where it comes first), so nothing here
+                // branches on a lane's own state.
+                constexpr int NONE = 64 * P2GO_PLANE;
                 const int here = lj * TK + lk;
                 auto place = [&](const P2GRole& r) -> int {
-                    const int ci = li - r.ox, cj = lj - r.oy, ck = lk - r.oz;
+                    const int ci = li - r.ox, cj = lj - r.oy;
                     const bool in_tile = ci >= 0 && ci < planes && cj >= 0 && cj < TJ;  // warp-uniform
                     const int c = ((ci & 3) * 16 + 2 * r.lane) * P2GO_PLANE + here - r.oy * TK - r.oz;
-                    return in_tile && (unsigned)ck < (unsigned)TK && n > 0 ? c : -1;
+                    return in_tile && (unsigned)(lk - r.oz) < (unsigned)TK ? c : NONE;
                 };
                 f32x2 sv[6], sw[6];
                 p2g_unroll<6>([&](auto index) {
@@ -268,10 +283,8 @@ __device__ __forceinline__ void p2g_ordered_tile(float* smem, int tile, const P2
                         static_assert(r.lane >= 0, "every pair is two roles");
                         if constexpr (r.second) {
                             const int c = place(r);
-                            if (c >= 0) {
-                                v[H] = sums[c];
-                                w[H] = sums[c + P2GO_PLANE];
-                            }
+                            v[H] = sums[c];
+                            w[H] = sums[c + P2GO_PLANE];
                         }
                     });
                     sv[I] = pack2(v[0], v[1]);
@@ -287,6 +300,7 @@ __device__ __forceinline__ void p2g_ordered_tile(float* smem, int tile, const P2
                     __syncwarp();
                     const int q1 = min(begin + n, base + m) - base;
                     const float* bq = bp + shift;
+#pragma unroll 2
                     for (int q = max(begin, base) - base; q < q1; ++q) {
                         const float sx = bq[3 * q] * g.inv_dx, sy = bq[3 * q + 1] * g.inv_dx, sz = bq[3 * q + 2] * g.inv_dx;
                         const float v = bv[q];
@@ -319,24 +333,18 @@ __device__ __forceinline__ void p2g_ordered_tile(float* smem, int tile, const P2
                         }
                         // weights x * y * z, left to right; cell b - o has index 1 - o (1 is b, 2 is b + 1, 0 is b - 1)
                         const f32x2 vv = pack2(v, v);
-                        f32x2 xx[3], yy[3], zz[3];
-                        if constexpr (A != 2) {  // pairs along k
-#pragma unroll
-                            for (int a = A == 0 ? 0 : 1; a < 3; ++a) xx[a] = pack2(x[a], x[a]);
-#pragma unroll
-                            for (int a = A == 1 ? 0 : 1; a < 3; ++a) yy[a] = pack2(y[a], y[a]);
-                            zz[0] = pack2(z[1], z[2]);
-                        } else {  // pairs along j
-#pragma unroll
-                            for (int a = 1; a < 3; ++a) xx[a] = pack2(x[a], x[a]);
-                            yy[0] = pack2(y[1], y[2]);
-#pragma unroll
-                            for (int a = 0; a < 3; ++a) zz[a] = pack2(z[a], z[a]);
-                        }
+                        // pairs along k (j when the component's axis is k)
+                        const f32x2 zz = pack2(z[1], z[2]), yy = pack2(y[1], y[2]);
                         p2g_unroll<6>([&](auto index) {
                             constexpr int I = decltype(index)::value;
                             constexpr P2GRole r = p2g_pair_role<A>(I, 0);
-                            const f32x2 wgt = mul2(mul2(xx[1 - r.ox], A == 2 ? yy[0] : yy[1 - r.oy]), A == 2 ? zz[1 - r.oz] : zz[0]);
+                            f32x2 wgt;
+                            if constexpr (A != 2) {
+                                const float xy = x[1 - r.ox] * y[1 - r.oy];
+                                wgt = mul2(pack2(xy, xy), zz);
+                            } else {
+                                wgt = mul2(mul2(pack2(x[1 - r.ox], x[1 - r.ox]), yy), pack2(z[1 - r.oz], z[1 - r.oz]));
+                            }
                             sv[I] = add2(sv[I], mul2(wgt, vv), one);
                             sw[I] = add2(sw[I], wgt, one);
                         });
@@ -354,10 +362,8 @@ __device__ __forceinline__ void p2g_ordered_tile(float* smem, int tile, const P2
                         constexpr int H = decltype(half)::value;
                         constexpr P2GRole r = p2g_pair_role<A>(I, H);
                         const int c = place(r);
-                        if (c >= 0) {
-                            sums[c] = H ? hi2(sv[I]) : lo2(sv[I]);
-                            sums[c + P2GO_PLANE] = H ? hi2(sw[I]) : lo2(sw[I]);
-                        }
+                        sums[c] = H ? hi2(sv[I]) : lo2(sv[I]);
+                        sums[c + P2GO_PLANE] = H ? hi2(sw[I]) : lo2(sw[I]);
                     });
                 });
                 __syncwarp();  // the buffer is free again
@@ -423,10 +429,10 @@ __global__ void __launch_bounds__(P2GO_THREADS, 2)
 }
 
 // Planes per tile. A tile walks one or two planes of bins more than it has planes of cells, so long tiles do less in
-// all, but a tile is a chain of planes and a small grid needs its blocks (us with 4 / 8 / 16 planes: 64^3 34 / 52 /
-// 74, 96^3 148 / 134 / 153, 117 x 90 x 139 246 / 218 / 206, 256^3 1583 / 1301 / 1185).
+// all, but a tile is a chain of planes and a small grid needs its blocks (us with 4 / 8 / 16 planes, before the last
+// refinements: 64^3 34 / 52 / 74, 96^3 148 / 134 / 153, 117 x 90 x 139 246 / 218 / 206, 256^3 1583 / 1301 / 1185).
 constexpr i64 P2GO_MIN_CELLS = 1 << 17;
-static inline int p2g_ordered_planes(i64 cells) {
+__host__ __device__ __forceinline__ int p2g_ordered_planes(i64 cells) {
     return cells >= (1 << 23) ? 32 : cells >= 1200000 ? 16 : cells >= (1 << 19) ? 8 : 4;
 }
 
