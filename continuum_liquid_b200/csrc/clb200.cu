@@ -451,16 +451,31 @@ int clb_particle_update_tiled(float* particles, float* velocity, float* previous
     CLB_REQUIRE(particles && velocity && u && v && w && u_old && v_old && w_old && bin_offsets && bin_counts,
                 "particle_update_tiled: null pointer");
     CLB_REQUIRE(motion == nullptr || obstacle != nullptr, "particle_update_tiled: a motion needs an obstacle");
+    // few particles: the per-particle kernel, the same values (the records' 16-byte loads need aligned arrays)
+    const bool aligned = ((reinterpret_cast<uintptr_t>(particles) | reinterpret_cast<uintptr_t>(velocity)) & 15) == 0;
+    if (n < PUT_MIN_PARTICLES && aligned) {
+        const int blocks = blocks_for(n, PT);
+        if (motion)
+            k_particle_update<true><<<blocks, PT, 0, CLB_STREAM(stream)>>>(
+                particles, velocity, previous_out, u, v, w, u_old, v_old, w_old, obstacle, n, inv_dx, nx, ny, nz,
+                flip_ratio, dt, lower, upper_x, upper_y, upper_z, motion_of(motion));
+        else
+            k_particle_update<false><<<blocks, PT, 0, CLB_STREAM(stream)>>>(
+                particles, velocity, previous_out, u, v, w, u_old, v_old, w_old, obstacle, n, inv_dx, nx, ny, nz,
+                flip_ratio, dt, lower, upper_x, upper_y, upper_z);
+        CLB_LAUNCH_CHECK("k_particle_update");
+        return 0;
+    }
     int tiles_j = 0, tiles_k = 0;
     const int tiles = particle_update_tiles(nx, ny, nz, &tiles_j, &tiles_k);
     if (motion)
         k_particle_update_tiled<true><<<tiles, PUT_THREADS, PUT_SMEM, CLB_STREAM(stream)>>>(
             particles, velocity, previous_out, u, v, w, u_old, v_old, w_old, obstacle, bin_offsets, bin_counts, inv_dx,
-            nx, ny, nz, flip_ratio, dt, lower, upper_x, upper_y, upper_z, tiles_j, tiles_k, motion_of(motion));
+            nx, ny, nz, flip_ratio, dt, lower, upper_x, upper_y, upper_z, tiles_j, tiles_k, motion_of(motion), 1.0f);
     else
         k_particle_update_tiled<false><<<tiles, PUT_THREADS, PUT_SMEM, CLB_STREAM(stream)>>>(
             particles, velocity, previous_out, u, v, w, u_old, v_old, w_old, obstacle, bin_offsets, bin_counts, inv_dx,
-            nx, ny, nz, flip_ratio, dt, lower, upper_x, upper_y, upper_z, tiles_j, tiles_k, RigidMotion{});
+            nx, ny, nz, flip_ratio, dt, lower, upper_x, upper_y, upper_z, tiles_j, tiles_k, RigidMotion{}, 1.0f);
     CLB_LAUNCH_CHECK("k_particle_update_tiled");
     return 0;
 }
