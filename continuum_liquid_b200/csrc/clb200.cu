@@ -12,6 +12,7 @@
 #include "mg_sweep.cuh"
 #include "mg_half.cuh"
 #include "mg_cluster.cuh"
+#include "mg_coarse.cuh"
 #include "mg_tiles.cuh"
 #include "mg_level0.cuh"
 #include "batch.cuh"
@@ -65,6 +66,14 @@ static cudaError_t cluster_visit_attr_one() {
     return e != cudaSuccess ? e
                             : cudaFuncSetAttribute(k_cluster_visit<NS, KA, KB, H>,
                                                    cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+}
+template <bool H>
+static cudaError_t coarse_slabs_attr() {
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_coarse_slabs<H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBottomSmemLimit);
+    return e != cudaSuccess
+               ? e
+               : cudaFuncSetAttribute(k_coarse_slabs<H>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
 }
 template <bool H>
 static cudaError_t cluster_visit_attr() {
@@ -139,6 +148,8 @@ int clb_init(int device) {
     e = e != cudaSuccess ? e : rbgs_iter_attr<false, true>();
     e = e != cudaSuccess ? e : cluster_visit_attr<false>();
     e = e != cudaSuccess ? e : cluster_visit_attr<true>();
+    e = e != cudaSuccess ? e : coarse_slabs_attr<false>();
+    e = e != cudaSuccess ? e : coarse_slabs_attr<true>();
     e = e != cudaSuccess ? e : cudaFuncSetAttribute(k_bottom_visit<1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, bottom_max);
     e = e != cudaSuccess ? e : cudaFuncSetAttribute(k_bottom_visit<2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, bottom_max);
     e = e != cudaSuccess ? e : cudaFuncSetAttribute(k_bottom_visit<4, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, bottom_max);
@@ -1065,8 +1076,80 @@ int smooth(const LevelView& v, float delta, int iterations, cudaStream_t s, bool
     return 0;
 }
 
+extern "C++" {
+template <bool H>
+static int launch_coarse_slabs(const LevelView& v, bool along_j, int cs, float delta, int iterations, cudaStream_t s) {
+    const int n0 = along_j ? v.ny : v.nx, n1 = along_j ? v.nx : v.ny;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(cs);
+    cfg.blockDim = dim3(COARSE_SLAB_THREADS);
+    cfg.dynamicSmemBytes = coarse_slab_smem(cs, n0, n1, v.nz);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cs;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cs > 8) {  // above the portable size: schedulable on this device with all the memory a launch may ask for?
+        static const bool ok = [] {
+            cudaLaunchConfig_t most = {};
+            cudaLaunchAttribute dim;
+            dim.id = cudaLaunchAttributeClusterDimension;
+            dim.val.clusterDim.x = CLUSTER_MAX;
+            dim.val.clusterDim.y = 1;
+            dim.val.clusterDim.z = 1;
+            most.gridDim = dim3(CLUSTER_MAX);
+            most.blockDim = dim3(COARSE_SLAB_THREADS);
+            most.dynamicSmemBytes = kBottomSmemLimit;
+            most.attrs = &dim;
+            most.numAttrs = 1;
+            int clusters = 0;
+            const bool fits =
+                cudaOccupancyMaxActiveClusters(&clusters, k_coarse_slabs<H>, &most) == cudaSuccess && clusters >= 1;
+            (void)cudaGetLastError();
+            return fits;
+        }();
+        if (!ok) return 0;
+    }
+    cfg.numAttrs = g_use_pdl ? 2 : 1;
+    (void)cudaLaunchKernelEx(&cfg, k_coarse_slabs<H>, v.p, v.b, v.opc, v.mask, delta, iterations, n0, n1, v.nz,
+                             along_j, v.scale, cs);
+    return check_launch("k_coarse_slabs") ? -1 : 1;
+}
+}  // extern "C++"
+
+// The coarsest level on the slabs of a cluster (mg_coarse.cuh), or on one block when its slots fit one; returns 1 if it
+// launched, 0 if the caller must go on, -1 on error. More slabs cost nothing but their ghost planes (a full level of
+// 41 x 9 x 34, us an iteration: 0.46 on 8, 0.42 on 16; of 9 x 27 x 27 0.47, 0.41, 0.38 on 4, 8, 16), one block saves
+// the cluster barrier (8 x 8 x 46: 0.25, against 0.36 to 0.40 on 2 to 8).
+int coarse_slabs(const LevelView& v, float delta, int iterations, cudaStream_t s) {
+    if (!g_use_cluster || v.l0 || iterations < 1 || v.nx < 3 || v.ny < 3 || v.nz < 3) return 0;
+    const bool along_j = v.ny > v.nx;
+    const int n0 = along_j ? v.ny : v.nx, n1 = along_j ? v.nx : v.ny;
+    const i64 plane = (i64)(n1 - 2) * ((v.nz - 1) / 2);  // slots of a colour in a plane
+    for (int most = plane * (n0 - 2) <= COARSE_SLAB_THREADS ? 1 : CLUSTER_MAX; most > 0; most = most > 8 ? 8 : 0) {
+        const int cs = most < n0 - 2 ? most : n0 - 2;
+        if (plane * coarse_slab_planes(cs, n0) > COARSE_SLAB_THREADS ||
+            coarse_slab_smem(cs, n0, n1, v.nz) > kBottomSmemLimit)
+            return 0;
+        const int did = v.half ? launch_coarse_slabs<true>(v, along_j, cs, delta, iterations, s)
+                               : launch_coarse_slabs<false>(v, along_j, cs, delta, iterations, s);
+        if (did != 0) return did;
+    }
+    return 0;
+}
+
 int coarse_solve(const LevelView& v, float delta, int iterations, cudaStream_t s) {
+    const int slabs = coarse_slabs(v, delta, iterations, s);
+    if (slabs != 0) return slabs < 0 ? 1 : 0;
     const int C = v.nx * v.ny * v.nz;
+    // Planes too large for a slab: colour by colour over the whole GPU. One block would read the level from memory in
+    // every phase (9 x 77 x 77, an iteration: 2.7 us against 47 us).
+    if (g_use_cluster && C > COARSE_SMEM_CELLS && !v.l0 && tile_sweeps(v)) return smooth(v, delta, iterations, s, true);
     if (v.half) {  // checked to fit shared memory by check_hierarchy
         launch(1, COARSE_THREADS, coarse_smem_bytes(C), s)(k_coarse_solve<true, false, true>,
             v.p, v.b, nullptr, v.opc, v.mask, delta, iterations, v.nx, v.ny, v.nz, v.scale);
