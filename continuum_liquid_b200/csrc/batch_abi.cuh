@@ -75,6 +75,7 @@ int batch_bottom(const clb_batch* B, int level, int pre, int post, int coarse_it
     else if (ka <= 2 && kb <= 1) CLB_BB(2, 1);
     else if (ka <= 4 && kb <= 1) CLB_BB(4, 1);
     else if (ka <= 4 && kb <= 2) CLB_BB(4, 2);
+    else if (ka <= 8 && kb <= 2) CLB_BB(8, 2);
     else if (ka <= 8 && kb <= 4) CLB_BB(8, 4);
     else CLB_REQUIRE(false, "batch: bottom visit tiles (%d, %d) too large", ka, kb);
 #undef CLB_BB

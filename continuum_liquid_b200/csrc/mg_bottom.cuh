@@ -80,37 +80,43 @@ __device__ __forceinline__ int split_cell(int i, int j, int k, int nx, int ny, i
     return 1 + (((i + j + k) & 1) * nx * ny + i * ny + j) * half + ((k - 1) >> 1);
 }
 
-// Constants of one owned cell of the second-coarsest level: smem index, diagonal (<= 0: not updated;
-// -1 marks cells that are not fluid or slots without a cell) and delta^2 * b.
+// Constants of one owned cell of the second-coarsest level: smem index, 1 / diagonal (0: a fluid cell with diagonal 0,
+// not updated; -1: not fluid, or a slot without a cell) and delta^2 * b. The diagonal comes with the weights (one
+// 16-byte load). With more than four cells of a colour per thread (keep_rhs) delta^2 * b is formed again in every
+// sweep instead of kept, so that fewer of the owned cells spill (15 x 20 x 19 over 9 x 12 x 11, a visit: 33 us, 39
+// with both kept and every thread taking two cells of B in every phase).
 struct OwnedCell {
     int c;
-    float d;
-    float r;  // 1 / d
+    float r;
     float d2b;
 };
+__host__ __device__ constexpr bool keep_rhs(int KA) { return KA <= 4; }
 
 // Owned coarsest-level cell with its neighbour weights in registers (constant for the whole visit).
 struct OwnedCellW {
-    int c, n;    // split_cell of the cell, and its slot in the other colour
+    int c;       // split_cell of the cell
     int zp, zm;  // split cells of its neighbours along k
     float d, r, d2b;
     float wxp, wxm, wyp, wym, wzp, wzm;
 };
 
-// sx, sy: split-layout strides along i and j.
-__device__ __forceinline__ float relaxed_w(const OwnedCellW& o, const float* sp, int sx, int sy) {
-    const float ws = o.wxp * sp[o.n + sx] + o.wxm * sp[o.n - sx] + o.wyp * sp[o.n + sy] + o.wym * sp[o.n - sy] +
+// sx, sy: split-layout strides along i and j; other: words from a cell to its slot in the other colour.
+__device__ __forceinline__ float relaxed_w(const OwnedCellW& o, const float* sp, int other, int sx, int sy) {
+    const int n = o.c + other;
+    const float ws = o.wxp * sp[n + sx] + o.wxm * sp[n - sx] + o.wyp * sp[n + sy] + o.wym * sp[n - sy] +
                      o.wzp * sp[o.zp] + o.wzm * sp[o.zm];
     return divide_by(ws - o.d2b, o.d, o.r);
 }
 
 // One red-black update of an owned cell (multigrid.cl:225-229), p and weights in shared memory.
-__device__ __forceinline__ float relaxed(const OwnedCell& o, const float* sp, const float4* so, int sx, int sy) {
+template <bool KEEP>
+__device__ __forceinline__ float relaxed(const OwnedCell& o, const float* sp, const float4* so, const float* sb,
+                                         float d2, int sx, int sy) {
     const int c = o.c;
     const float4 self = so[c];
     const float ws = self.y * sp[c + sx] + so[c - sx].y * sp[c - sx] + self.z * sp[c + sy] + so[c - sy].z * sp[c - sy] +
                      self.w * sp[c + 1] + so[c - 1].w * sp[c - 1];
-    return divide_by(ws - o.d2b, o.d, o.r);
+    return divide_by(ws - (KEEP ? o.d2b : d2 * sb[c]), self.x, o.r);
 }
 
 // The updates of a warp's owned slots 0 .. active - 1 of one colour (active is the same in the whole warp), two
@@ -288,8 +294,8 @@ __device__ __forceinline__ void bottom_cells(const BottomSmem& S, BottomCells<KA
             const int c = r < S.count[colour] ? S.list_a[colour * la + r] : -1;
             OwnedCell& o = R.A[colour][m];
             o.c = c < 0 ? (any + 1) * anz + 1 : c;  // a slot without a cell loads an interior cell and stores nothing
-            o.d = c < 0 ? -1.0f : S.soa[c].x;       // fluid: >= 0
-            o.r = 1.0f / o.d;
+            const float d = c < 0 ? -1.0f : S.soa[c].x;  // fluid: >= 0
+            o.r = d > 0.0f ? 1.0f / d : d < 0.0f ? -1.0f : 0.0f;
             o.d2b = 0.0f;
         }
 #pragma unroll
@@ -300,16 +306,15 @@ __device__ __forceinline__ void bottom_cells(const BottomSmem& S, BottomCells<KA
             const int c = r < S.count[2 + colour] ? S.list_b[colour * lb + r] : -1;
             OwnedCellW& o = R.B[colour][m];
             o.d2b = 0.0f;
-            o.c = o.zp = o.zm = 0;
-            o.n = 1 + bny * ((bnz - 1) / 2);  // a slot without a cell loads some cells and stores nothing
+            o.zp = o.zm = 0;
+            o.c = 1 + (colour * bnx + 1) * bny * ((bnz - 1) / 2);  // a slot without a cell loads some cells, stores nothing
             o.d = o.r = -1.0f;
             o.wxp = o.wxm = o.wyp = o.wym = o.wzp = o.wzm = 0.0f;
             if (c >= 0) {
                 const float4 self = S.sob[c];
                 const int i = c / bsx, j = (c / bsy) % bny, k = c % bnz;
                 o.c = split_cell(i, j, k, bnx, bny, bnz);
-                o.n = o.c + (((i + j + k) & 1) ? -1 : 1) * bnx * bny * ((bnz - 1) / 2);
-                const int up = o.n + ((k - 1) & 1);
+                const int up = o.c + (colour ? -1 : 1) * bnx * bny * ((bnz - 1) / 2) + ((k - 1) & 1);
                 o.zp = k + 1 <= bnz - 2 ? up : 0;
                 o.zm = k > 1 ? up - 1 : 0;
                 o.d = self.x;
@@ -332,7 +337,7 @@ __device__ __forceinline__ void bottom_rhs(const BottomSmem& S, BottomCells<KA, 
 #pragma unroll
         for (int m = 0; m < KA; ++m) {
             OwnedCell& o = R.A[colour][m];
-            o.d2b = o.d < 0.0f ? 0.0f : d2 * S.sba[o.c];
+            if (keep_rhs(KA)) o.d2b = o.r < 0.0f ? 0.0f : d2 * S.sba[o.c];
         }
 }
 
@@ -367,9 +372,9 @@ __device__ __forceinline__ void bottom_core(const BottomSmem& S, BottomCells<KA,
 #pragma unroll
             for (int colour = 0; colour < 2; ++colour) {
                 relax_slots<KA>(
-                    aslots[colour], [&](int m) { return relaxed(A[colour][m], spa, soa, asx, asy); },
+                    aslots[colour], [&](int m) { return relaxed<keep_rhs(KA)>(A[colour][m], spa, soa, sba, d2, asx, asy); },
                     [&](int m, float v) {
-                        if (A[colour][m].d > 0.0f) spa[A[colour][m].c] = v;
+                        if (A[colour][m].r > 0.0f) spa[A[colour][m].c] = v;
                     });
                 __syncthreads();
             }
@@ -431,16 +436,17 @@ __device__ __forceinline__ void bottom_core(const BottomSmem& S, BottomCells<KA,
     if ((int)(threadIdx.x >> 5) < bwarps) {
         // two coarse solves of the W (multigrid.py:127-170; b_solves: one when the coarsest level is
         // visited once), pre + coarse_iters iterations each
-        const int iterations = b_solves * (pre + coarse_iters), sx = bny * half, sy = half;
+        const int bslots[2] = {active_slots(S.count[2], BOTTOM_THREADS), active_slots(S.count[3], BOTTOM_THREADS)};
+        const int iterations = b_solves * (pre + coarse_iters), sx = bny * half, sy = half, other = bnx * sx;
         for (int it = 0; it < iterations; ++it)
 #pragma unroll
             for (int colour = 0; colour < 2; ++colour) {
-                float v[MB];
-#pragma unroll
-                for (int m = 0; m < MB; ++m) v[m] = relaxed_w(B[colour][m], spb, sx, sy);
-#pragma unroll
-                for (int m = 0; m < MB; ++m)
-                    if (B[colour][m].d > 0.0f) spb[B[colour][m].c] = v[m];
+                auto put = [&](int m, float v) {
+                    if (B[colour][m].d > 0.0f) spb[B[colour][m].c] = v;
+                };
+                auto value = [&](int m) { return relaxed_w(B[colour][m], spb, colour ? -other : other, sx, sy); };
+                if (MB == 1) put(0, value(0));
+                else relax_slots<MB>(bslots[colour], value, put);
                 bar_b(bwarps);
             }
     }
@@ -450,7 +456,7 @@ __device__ __forceinline__ void bottom_core(const BottomSmem& S, BottomCells<KA,
     for (int colour = 0; colour < 2; ++colour)
 #pragma unroll
         for (int m = 0; m < KA; ++m) {
-            if (A[colour][m].d < 0.0f) continue;  // interior fluid cells only
+            if (A[colour][m].r < 0.0f) continue;  // interior fluid cells only
             const int c = A[colour][m].c;
             const int i = c / asx, j = (c / asy) % any, k = c % anz;
             const int I = min((i - 1) / 2 + 1, bnx - 2), J = min((j - 1) / 2 + 1, bny - 2),
