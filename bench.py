@@ -721,6 +721,13 @@ def pressure_error_audit(sim, snapshot, end_positions, steps, min_size):
             "replay_bit_exact": replay_exact}
 
 
+def p2g_kernel(tiled, cells):
+    """The P2G kernel a step launches (csrc/p2g_tiled.cuh P2GT_MIN_CELLS, csrc/p2g_ordered.cuh P2GO_MIN_CELLS)."""
+    if tiled and cells >= 3_500_000:
+        return "k_p2g_tiled"
+    return "k_p2g_ordered" if cells >= 1 << 17 else "k_p2g_gather"
+
+
 def kernel_rooflines(sim, peak, ms_per_step, reps=5):
     """Device time of each particle stage launched alone (CUDA events on the launching stream, the mean
     of ``reps`` launches on the scene's current state) against its algorithmic bytes."""
@@ -760,7 +767,7 @@ def kernel_rooflines(sim, peak, ms_per_step, reps=5):
     timed("sort", "k_scatter_perm + k_stable_gather", 56 * n + 4 * C,
           lambda: pm.sort_particles(k, None, pos, vel, sim.particle_work, sim.particle_velocity_work,
                                     sim.scan_outputs[0], sim.bin_counts, scratch, n))
-    timed("p2g", "k_p2g_tiled" if tiled else "k_p2g_gather", 24 * n + 24 * C,
+    timed("p2g", p2g_kernel(tiled, C), 24 * n + 24 * C,
           lambda: pm.particle_to_grid_gather(k, None, sim.particle_work, sim.particle_velocity_work,
                                              sim.scan_outputs[0], sim.bin_counts, (sim.u, sim.v, sim.w),
                                              sim.fluid_fraction, gs, sim.dx, sim.particles_per_cell, tiled=tiled))
@@ -1167,8 +1174,7 @@ def our_arm(args):
         solver_info = {"pressure": solver_description(args.method, sim.options.pre_smooth, sim.options.post_smooth,
                                                       sim.options.coarse_iterations, fp16_levels, single_from,
                                                       sim.options.prolong_scale, sim.options.coarse_smooth),
-                       "p2g": "tiled scatter (k_p2g_tiled)" if sim.options.tiled_p2g() else
-                              "reference-order gather (k_p2g_gather)",
+                       "p2g": p2g_kernel(sim.options.tiled_p2g(), int(np.prod(sim.grid_shape))),
                        "multigrid_levels": [list(s) for s in h.shapes], "sweep_kinds": h.sweeps(),
                        "sweep_tuning_ms_per_iteration": h.tuning}
         line = {

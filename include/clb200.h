@@ -100,7 +100,8 @@ int clb_particle_to_grid(const float* particles, const float* velocity, float* p
  * scatter that visits each particle once (the tolerance-mode path). Every weight is the reference's;
  * the sums of a cell are added in a different (fixed) order, so velocities agree with
  * clb_particle_to_grid_gather to float rounding (not bit for bit); the fluid fraction is identical
- * and a face that no particle weighs is 0 in both. Deterministic: the same inputs give the same bits on every run. */
+ * and a face that no particle weighs is 0 in both. Grids below 3.5M cells take the reference's order (the faster
+ * kernel there). Deterministic: the same inputs give the same bits on every run. */
 int clb_particle_to_grid_gather_tiled(const float* particles, const float* velocity, const int32_t* bin_offsets,
                                       const int32_t* bin_counts, float* u, float* v, float* w, float* fluid_fraction,
                                       float inv_dx, float inv_particles_per_cell, int nx, int ny, int nz,
@@ -196,7 +197,8 @@ int clb_particle_obstacle_bc_moving(float* particles, const float* previous, flo
  * form below; motion as there) walking the bins of 8 x 8 x 30-bin tiles: particles must be sorted by
  * bin, bin_offsets / bin_counts describing them (the counting sort of clb_particle_to_grid, before any
  * particle moves). Each block stages the six grid arrays its bins' particles sample in shared memory.
- * The same values as clb_particle_update, bit for bit. */
+ * Below 2.3M particles (16-byte aligned arrays) the per-particle kernel runs instead. The same values as
+ * clb_particle_update, bit for bit. */
 int clb_particle_update_tiled(float* particles, float* velocity, float* previous_out, const float* u, const float* v,
                               const float* w, const float* u_old, const float* v_old, const float* w_old,
                               const uint8_t* obstacle, const int32_t* bin_offsets, const int32_t* bin_counts,
@@ -465,11 +467,11 @@ int clb_tc_test_gemm(const void* a, const void* b, float* c, int M, int N, int K
  *  arrange_weights: wf[cout][kpad] (forward) and, when wd != NULL, wd[cin][kpad2] (data grad), BF16,
  *                   kpad >= 27*cin and kpad2 >= 27*cout multiples of 64, zero-padded.
  *  forward:  y = act(bias + conv(x)), cin % 8 == 0, cout in {16, 32, 64}, relu = 0/1; bias (nullable)
- *            16-byte aligned. Forward and data gradient stage an input tile in shared memory and read
- *            each tap as a shifted window of it (no per-tap gather).
+ *            16-byte aligned. Forward and data gradient stage each input slice of a tile in shared memory
+ *            once and read the taps as shifted windows of it.
  *  dgrad:    dx = conv^T(dy) * (mask_x > 0) (mask_x nullable), cout % 8 == 0, cin in {16,32,48,64,96}.
  *  wgrad:    dw[27*cin][cout] += sum over voxels (FP32 atomics; zero dw first), cout in {16, 32, 64};
- *            each block reduces chunks_per_block chunks of 64 voxels. */
+ *            no tensor-core sum is longer than chunks_per_block chunks of 64 voxels. */
 int clb_conv3d_arrange_weights(const float* w, void* wf, void* wd, int cin, int cout, int kpad, int kpad2,
                                void* stream);
 int clb_conv3d_forward(const void* x, const void* wf, const float* bias, void* y, int B, int D, int H, int W, int cin,
