@@ -169,6 +169,7 @@ __global__ void __launch_bounds__(COARSE_SLAB_THREADS, 1)
                 if (o.first) left[o.c] = v;
                 if (o.last) right[o.c] = v;
             }
+            __syncwarp();  // the barriers are taken by whole warps
             if (cs > 1) cluster_barrier();
             else bar_b(warps);
         }
