@@ -89,9 +89,9 @@ static cudaError_t conv_march_attr() {
     return conv::conv_march_run<N, DG>(true, nullptr, nullptr, nullptr, nullptr, nullptr, conv::Vol{}, 0, 0, 0, false,
                                        conv::MarchPlan{}, nullptr);
 }
-template <int NC>
+template <int NC, bool FINE>
 static cudaError_t conv_wgrad_attr() {
-    return cudaFuncSetAttribute(conv::k_conv_wgrad_march<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    return cudaFuncSetAttribute(conv::k_conv_wgrad_march<NC, FINE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 conv::CM_SMEM_LIMIT);
 }
 static int conv_set_attributes() {
@@ -104,8 +104,9 @@ static int conv_set_attributes() {
     e = e != cudaSuccess ? e : conv_march_attr<48, true>();
     e = e != cudaSuccess ? e : conv_march_attr<64, true>();
     e = e != cudaSuccess ? e : conv_march_attr<96, true>();
-    e = e != cudaSuccess ? e : conv_wgrad_attr<16>();
-    e = e != cudaSuccess ? e : conv_wgrad_attr<32>();
+    e = e != cudaSuccess ? e : conv_wgrad_attr<16, false>();
+    e = e != cudaSuccess ? e : conv_wgrad_attr<16, true>();
+    e = e != cudaSuccess ? e : conv_wgrad_attr<32, false>();
     return check_call(e, "convolution attributes");
 }
 
@@ -1798,10 +1799,12 @@ int clb_conv3d_wgrad(const void* x, const void* dy, float* dw, int B, int D, int
     cudaStream_t s = CLB_STREAM(stream);
     const auto* X = (const __nv_bfloat16*)x;
     const auto* DY = (const __nv_bfloat16*)dy;
-    if (cout == 16)
-        conv::k_conv_wgrad_march<16><<<pl.grid, conv::WG_THREADS, pl.smem, s>>>(X, DY, dw, g, cin, cout, pl);
+    if (pl.fine)
+        conv::k_conv_wgrad_march<16, true><<<pl.grid, conv::WG_THREADS, pl.smem, s>>>(X, DY, dw, g, cin, cout, pl);
+    else if (pl.nc == 16)
+        conv::k_conv_wgrad_march<16, false><<<pl.grid, conv::WG_THREADS, pl.smem, s>>>(X, DY, dw, g, cin, cout, pl);
     else
-        conv::k_conv_wgrad_march<32><<<pl.grid, conv::WG_THREADS, pl.smem, s>>>(X, DY, dw, g, cin, cout, pl);
+        conv::k_conv_wgrad_march<32, false><<<pl.grid, conv::WG_THREADS, pl.smem, s>>>(X, DY, dw, g, cin, cout, pl);
     CLB_LAUNCH_CHECK("k_conv_wgrad_march");
     return 0;
 }
