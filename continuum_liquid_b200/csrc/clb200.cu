@@ -91,8 +91,11 @@ static cudaError_t conv_march_attr() {
 }
 template <int NC, bool FINE>
 static cudaError_t conv_wgrad_attr() {
-    return cudaFuncSetAttribute(conv::k_conv_wgrad_march<NC, FINE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                conv::CM_SMEM_LIMIT);
+    cudaError_t e = cudaSuccess;
+    for (auto* k : {conv::k_conv_wgrad_march<NC, FINE, 0>, conv::k_conv_wgrad_march<NC, FINE, 1>,
+                    conv::k_conv_wgrad_march<NC, FINE, 2>})
+        e = e != cudaSuccess ? e : cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, conv::CM_SMEM_LIMIT);
+    return e;
 }
 static int conv_set_attributes() {
     cudaError_t e = cudaSuccess;
@@ -1799,12 +1802,21 @@ int clb_conv3d_wgrad(const void* x, const void* dy, float* dw, int B, int D, int
     cudaStream_t s = CLB_STREAM(stream);
     const auto* X = (const __nv_bfloat16*)x;
     const auto* DY = (const __nv_bfloat16*)dy;
-    if (pl.fine)
-        conv::k_conv_wgrad_march<16, true><<<pl.grid, conv::WG_THREADS, pl.smem, s>>>(X, DY, dw, g, cin, cout, pl);
-    else if (pl.nc == 16)
-        conv::k_conv_wgrad_march<16, false><<<pl.grid, conv::WG_THREADS, pl.smem, s>>>(X, DY, dw, g, cin, cout, pl);
-    else
-        conv::k_conv_wgrad_march<32, false><<<pl.grid, conv::WG_THREADS, pl.smem, s>>>(X, DY, dw, g, cin, cout, pl);
+#define CLB_WG_EDGE(NC, FINE, EDGE) \
+    conv::k_conv_wgrad_march<NC, FINE, EDGE><<<pl.grid, conv::WG_THREADS, pl.smem, s>>>(X, DY, dw, g, cin, cout, pl)
+#define CLB_WG(NC, FINE)                              \
+    if (pl.over == 0) CLB_WG_EDGE(NC, FINE, 0);       \
+    else if (pl.over <= 8) CLB_WG_EDGE(NC, FINE, 1);  \
+    else CLB_WG_EDGE(NC, FINE, 2)
+    if (pl.fine) {
+        CLB_WG(16, true);
+    } else if (pl.nc == 16) {
+        CLB_WG(16, false);
+    } else {
+        CLB_WG(32, false);
+    }
+#undef CLB_WG
+#undef CLB_WG_EDGE
     CLB_LAUNCH_CHECK("k_conv_wgrad_march");
     return 0;
 }

@@ -23,6 +23,14 @@
 // 2.3e-7 with the additions to dw, 1.9e-7 in the form that gathers every tap's operand.
 // Rows of the operand beyond the three dy taps read whatever lies there and feed accumulator rows nobody reads.
 //
+// Where W is no multiple of 16 the last tile has `over` columns, and the others of its dy are zeros. A zero times an
+// infinite x is not zero, so their x has to be finite: zeros beyond W, except in the tap that looks back along x, where
+// the first of them meets column W - 1. That tap's K group of eight columns is replaced there (back): over = 8 takes
+// zeros; over < 8 needs no second group at all (zeros for every tap), and so leaves room for a copy of the first eight
+// columns without column W - 1; over > 8 (EDGE 2) stages a copy of the second eight in eight more cells a row. The zeros
+// lie behind the slots, reached by the K groups' stride, which shrinks as the start moves on. 64 -> 64, us: 8 x 50^3
+// 453 (437 without this), 4 x 60^3 (EDGE 2) 330 (285).
+//
 // Measured (B200, 8 x 64^3, us; the form that gathered every tap's operand per block of voxels): 8 -> 16 126 (440),
 // 16 -> 16 125 (907), 32 -> 32 170 (1840), 48 -> 16 248 (2758), 32 -> 64 322 (2447), 96 -> 32 485 (6125),
 // 64 -> 64 644 (4861). The MMAs' fixed 46 cycles bound it now (16 -> 16: 3 per 16 voxels and 8 / 7 of the slices
@@ -39,6 +47,7 @@ namespace conv {
 constexpr int WG_STG = 8, WG_FLUSH = 8;
 constexpr int WG_THREADS = 32 * (WG_STG + WG_FLUSH + 1);
 constexpr int WG_T = 16, WG_RW = WG_T + 2;  // rows and columns of a tile, with halo
+constexpr int WG_WIDE = WG_RW + 8;          // cells of a staged row that also holds a copy of eight columns
 constexpr int WG_MAX_STAGES = 6;
 constexpr int WG_CI = 32;                   // input channels per block, at most
 constexpr int WG_FINE = 8;                  // chunks of 64 voxels a sum below which FINE runs
@@ -49,6 +58,7 @@ struct WgradPlan {
     int stages, x_bytes, g_bytes;  // x slices in the ring, bytes of one; bytes of the dy buffer (2 Lz slices)
     int flush, flush_rows;         // slices between flushes; FINE: rows (WG_T: a slice)
     int fine, nc;
+    int over;  // W % 16
     int vec;                       // dw is 16-byte aligned
     int smem, tmem_cols;
     i64 tiles;
@@ -56,15 +66,18 @@ struct WgradPlan {
 };
 
 // NC: output channels of the block (16 or 32). FINE: short sums, added up in registers (16 output channels: 80 a thread).
-template <int NC, bool FINE>
+// EDGE: 0 where W is a multiple of 16, 1 where its last tile has up to 8 columns, 2 where it has more.
+template <int NC, bool FINE, int EDGE>
 __global__ void __launch_bounds__(WG_THREADS, 1)
     k_conv_wgrad_march(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
                        float* __restrict__ dw, Vol g, int Cin, int Cout, WgradPlan pl) {
     using namespace tc;
     static_assert(!FINE || NC == 16, "the registers of a flushing thread hold 16 output channels");
+    constexpr bool RAGGED = EDGE > 0;
+    constexpr int rw = EDGE == 2 ? WG_WIDE : WG_RW;
     constexpr int NPG = NC / 8, N3 = 3 * NC, COLS = 3 * N3;
     constexpr int SETS = FINE ? 2 : 1;  // of accumulators: short sums are taken while the next are formed
-    constexpr int ST = 32 * WG_STG, NEX = (WG_RW * WG_RW * (WG_CI / 8) + ST - 1) / ST, NEG = WG_T * WG_T * NPG / ST;
+    constexpr int ST = 32 * WG_STG, NEX = (WG_RW * rw * (WG_CI / 8) + ST - 1) / ST, NEG = WG_T * WG_T * NPG / ST;
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t full[WG_MAX_STAGES], empty[WG_MAX_STAGES], acc_full[2], acc_free[2];
     __shared__ uint32_t tmem_slot;
@@ -75,6 +88,13 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
     const int ci0 = (job % pl.ci_chunks) * WG_CI, co0 = (job / pl.ci_chunks) * NC;
     const int np = min(WG_CI, Cin - ci0) / 8;
     const int S = pl.stages, slots = 2 * pl.Lz;
+    const uint32_t xs = smem_u32(smem) + (uint32_t)pl.g_bytes, gs = smem_u32(smem);
+    const uint32_t zeros = xs + (uint32_t)(S * pl.x_bytes);  // 16 rows of rw cells
+    if (EDGE == 1) {
+        for (int c = threadIdx.x; c < 16 * rw; c += WG_THREADS)
+            reinterpret_cast<uint4*>(smem + pl.g_bytes + S * pl.x_bytes)[c] = make_uint4(0u, 0u, 0u, 0u);
+        fence_proxy_async();
+    }
     if (threadIdx.x == 0) {
         for (int s = 0; s < WG_MAX_STAGES; ++s) {
             mbar_init(&full[s], WG_STG);
@@ -144,7 +164,6 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
             par ^= 1u;
         }
     };
-    const uint32_t xs = smem_u32(smem) + (uint32_t)pl.g_bytes, gs = smem_u32(smem);
 
     if (warp == WG_STG + WG_FLUSH) {
         const bool leader = elect_one();
@@ -157,9 +176,9 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
             const uint32_t idesc = instr_desc(TC_M, (g1 - g0 + 1) * NC, true, true);
             const int slot0 = (at.k & 1) * pl.Lz + at.i - 2 + g0;
             uint32_t dcol = tmem + (uint32_t)((flushes % SETS) * COLS + g0 * NC);
-            uint64_t ad = smem_desc(xs + (uint32_t)(s * pl.x_bytes), 128u, (uint32_t)WG_RW * 16u);
+            const uint32_t x0 = xs + (uint32_t)(s * pl.x_bytes), xrow = (uint32_t)rw * 16u;
             uint64_t bd = smem_desc(gs + (uint32_t)(slot0 * NPG) * 256u, 128u, 256u);
-            const uint64_t astep = (uint64_t)(np * WG_RW), bstep = (uint64_t)(slots * NPG * 16);
+            const uint64_t astep = (uint64_t)(np * rw), bstep = (uint64_t)(slots * NPG * 16);
             const int rows = min(WG_T, g.H - at.y0);
             auto flush = [&]() {  // ends the sums of a set; returns once the next set's last ones are taken
                 if (leader) mma_commit(&acc_full[flushes % SETS]);
@@ -170,23 +189,44 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
                 if (FINE) dcol = tmem + (uint32_t)((flushes % SETS) * COLS + g0 * NC);
                 return true;
             };
-            auto row = [&]() {
+            // the slice's rows: the taps from ad, the one that looks back from `back` (LAST: the overhanging tile)
+            auto slice = [&](auto last, uint64_t ad, uint64_t ad_step, uint64_t back, uint64_t back_step) {
+                constexpr bool LAST = decltype(last)::value;
+                auto row = [&]() {
 #pragma unroll
-                for (int dx = 0; dx < 3; ++dx)
-                    if (leader) mma_bf16(dcol + (uint32_t)(dx * N3), ad + (uint64_t)dx, bd, idesc, 1u);
-                ad += astep;
-                bd += bstep;
-            };
-            bool ok = true;
-            if constexpr (FINE) {
-                for (int y = 0;;) {
+                    for (int dx = 0; dx < 3; ++dx)
+                        if (leader)
+                            mma_bf16(dcol + (uint32_t)(dx * N3), LAST && dx == 0 ? back : ad + (uint64_t)dx, bd, idesc, 1u);
+                    ad += ad_step;
+                    if (LAST) back += back_step;
+                    bd += bstep;
+                };
+                if constexpr (FINE) {
+                    for (int y = 0;;) {
 #pragma unroll 4
-                    for (const int end = min(rows, y + pl.flush_rows); y < end; ++y) row();
-                    if (y == rows || !(ok = flush())) break;
+                        for (const int end = min(rows, y + pl.flush_rows); y < end; ++y) row();
+                        if (y == rows) return true;
+                        if (!flush()) return false;
+                    }
+                } else {
+#pragma unroll 4
+                    for (int y = 0; y < rows; ++y) row();
+                    return true;
                 }
+            };
+            bool ok;
+            const uint64_t plain = smem_desc(x0, 128u, xrow);
+            if (RAGGED && at.x0 + WG_T > g.W) {
+                const uint64_t to_zeros = astep - (astep << 16);  // the start moves on, start + stride stays
+                if (EDGE == 1 && pl.over < 8)
+                    ok = slice(std::true_type{}, smem_desc(x0, zeros - x0, xrow), to_zeros,
+                               smem_desc(x0 + 160u, zeros - x0 - 160u, xrow), to_zeros);
+                else if (EDGE == 1)
+                    ok = slice(std::true_type{}, plain, astep, smem_desc(x0, zeros - x0, xrow), to_zeros);
+                else
+                    ok = slice(std::true_type{}, plain, astep, smem_desc(x0, (uint32_t)WG_RW * 16u, xrow), astep);
             } else {
-#pragma unroll 4
-                for (int y = 0; y < rows; ++y) row();
+                ok = slice(std::false_type{}, plain, astep, plain, astep);
             }
             if (leader) mma_commit(&empty[s]);
             __syncwarp();
@@ -204,7 +244,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
         uint32_t xin = 0, gin = 0;
         i64 mapped = -1;
         bool ok = true;
-        const int xpieces = WG_RW * WG_RW * np, nex = (xpieces + ST - 1) / ST;
+        const int xpieces = WG_RW * rw * np, nex = (xpieces + ST - 1) / ST;
         const i64 xslice = (i64)g.H * g.W * Cin, gslice = (i64)g.H * g.W * Cout;
         const int lag = S >= 6 ? 3 : S >= 4 ? 2 : 1;
         int announce_s = 0, ahead = 0;
@@ -223,10 +263,21 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
 #pragma unroll
                 for (int e = 0; e < NEX; ++e) {
                     const int f = min(tid + e * ST, xpieces - 1);
-                    const int p = f % np, pos = f / np, row = pos / WG_RW, col = pos - row * WG_RW;
+                    const int p = f % np, pos = f / np, row = pos / rw, cell = pos - row * rw;
+                    int col = cell, end = WG_RW;  // a cell's column, and the first one that it leaves out
+                    if (EDGE) {
+                        const bool last = at.x0 + WG_T > g.W;
+                        if (EDGE == 1 && last && pl.over < 8 && cell >= 10) {  // the copy of columns 0 .. 7
+                            col = cell - 10;
+                            end = pl.over;
+                        } else if (EDGE == 2 && cell >= WG_RW) {  // the copy of columns 8 .. 15
+                            col = cell - WG_RW + 8;
+                            end = last ? pl.over : 0;
+                        }
+                    }
                     const int gy = at.y0 + row - 1, gx = at.x0 + col - 1;
-                    const bool in = gy >= 0 && gy < g.H && gx >= 0 && gx < g.W;
-                    xdst[e] = (uint32_t)((row * np + p) * WG_RW + col) * 16u;
+                    const bool in = gy >= 0 && gy < g.H && gx >= 0 && gx < g.W && col < end;
+                    xdst[e] = (uint32_t)((row * np + p) * rw + cell) * 16u;
                     xoff[e] = in ? ((uint32_t)gy * (uint32_t)g.W + (uint32_t)gx) * (uint32_t)(Cin / 8) + (uint32_t)p : 0u;
                     xin |= in ? 1u << e : 0u;
                 }
@@ -364,7 +415,9 @@ static inline bool wgrad_plan(int B, int D, int H, int W, int Cin, int Cout, int
     p.ci_chunks = (Cin + WG_CI - 1) / WG_CI;
     p.co_chunks = Cout / NC;
     const int jobs = p.ci_chunks * p.co_chunks;
-    p.x_bytes = WG_RW * WG_RW * npx * 16;
+    p.over = W % WG_T;
+    const int rw = p.over > 8 ? WG_WIDE : WG_RW;
+    p.x_bytes = WG_RW * rw * npx * 16;
     // 4 chunks of 64 voxels: one slice of 16 x 16
     p.fine = fine ? 1 : 0;
     p.nc = NC;
@@ -372,7 +425,7 @@ static inline bool wgrad_plan(int B, int D, int H, int W, int Cin, int Cout, int
     p.flush_rows = chunks_per_block < 4 ? 4 * chunks_per_block : WG_T;
     p.vec = aligned ? 1 : 0;
     p.tmem_cols = NC == 16 && !fine ? 256 : 512;
-    const int tail = 16 * WG_RW * 16;  // operand rows past the last slot's end are read (and dropped)
+    const int tail = 16 * rw * 16;  // operand rows past the last slot's end are read (and dropped); EDGE 1: zeros
     const int per_job = sms / jobs > 0 ? sms / jobs : 1;
     double best_cost = -1.0;
     for (int Lz = D < 16 ? D : 16; Lz >= 1; --Lz) {
