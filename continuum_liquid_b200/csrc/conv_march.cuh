@@ -21,7 +21,8 @@
 // Blocks are persistent; weights stay in shared memory unless
 // they do not fit, in which case the source channels go in passes of KC channels with double-buffered weights.
 // An 8-channel source (the first layer) pairs neighbouring taps in one K = 16 step instead of padding
-// with zeros: the second tap's channels are "LBO" bytes further in the same plane.
+// with zeros: the second tap's channels are "LBO" bytes further in the same plane. The ninth tap's pair is a plane of
+// zeros behind the slots (a tap again with weight 0 would turn an infinite activation into NaN).
 //
 // Measured (B200, 128^3, us; the same layers with one MMA per tap, N = Cout, and three slices staged per output
 // slice): 8 -> 16 49 (128), 16 -> 16 64 (148), 32 -> 32 132 (548), 48 -> 16 138 (723), 96 -> 32 367 (1501),
@@ -57,6 +58,9 @@ struct MarchPlan {
     int tmem_cols, smem, grid;
     i64 tiles;
 };
+
+// The zeros an 8-channel source's ninth tap is paired with: what the 16 rows and nx8 tiles of an operand reach.
+__host__ __device__ constexpr int cm_zero_bytes(int nx8) { return (15 * (8 * nx8 + 2) + 8 * nx8) * 16; }
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0)
@@ -150,6 +154,12 @@ __global__ void __launch_bounds__(CM_THREADS, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
+    const uint32_t zeros = smem_u32(slots) + (uint32_t)(pl.stages * pl.slot_bytes);
+    if (PAIRS) {
+        for (int t = threadIdx.x; t < cm_zero_bytes(NX8) / 16; t += CM_THREADS)
+            reinterpret_cast<uint4*>(slots + pl.stages * pl.slot_bytes)[t] = make_uint4(0u, 0u, 0u, 0u);
+        fence_proxy_async();
+    }
     if (warp < 4) {  // accumulators start at zero; the epilogue leaves them at zero for the next tile
         for (int c = 0; c < pl.tmem_cols; c += 16) tmem_st16_zero(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c);
         tmem_wait_st();
@@ -177,11 +187,11 @@ __global__ void __launch_bounds__(CM_THREADS, 1)
         for (int t = tid; t < count; t += threads) {  // (unit, K group, output slice, n)
             const int n3 = t % N3, r = t / N3, kg = r & 1, q = r >> 1;
             const int gq = n3 / N, co = n3 - gq * N;
-            const int u = PAIRS ? 2 * q + kg - (q == 4 ? 1 : 0) : q % 9;
+            const int u = PAIRS ? (q < 4 ? 2 * q + kg : 8) : q % 9;
             const int c = PAIRS ? 0 : c0 + 16 * (q / 9) + 8 * kg;
             // the unit's shift reads source voxel v + (dy, dx); slice z feeds output z - 1 + gq
             const int tap = DGRAD ? gq * 9 + (8 - u) : (2 - gq) * 9 + u;
-            const bool in = PAIRS ? !(q == 4 && kg == 0) : c < Cs;
+            const bool in = PAIRS ? !(q == 4 && kg == 1) : c < Cs;
             cp_async16(w0 + (uint32_t)t * 16u, in ? wmat + (i64)co * Kpad + tap * Cs + c : wmat, in);
         }
     };
@@ -228,13 +238,13 @@ __global__ void __launch_bounds__(CM_THREADS, 1)
                 }
             };
             if constexpr (PAIRS) {
-                // taps 2 q and 2 q + 1 of the plane (q = 4: tap 7 again, times 0, and tap 8)
+                // taps 2 q and 2 q + 1 of the plane, tap 8 and the zeros
 #pragma unroll
                 for (int q = 0; q < 5; ++q) {
-                    const int u0 = q < 4 ? 2 * q : 7, u1 = u0 + 1;
+                    const int u0 = 2 * q, u1 = u0 + 1;
                     const int o0 = (u0 / 3) * RW + u0 % 3, o1 = (u1 / 3) * RW + u1 % 3;
-                    issue(smem_desc(slot, (uint32_t)(o1 - o0) * 16u, row_bytes) + (uint64_t)o0,
-                          b0 + (uint64_t)(q * 2 * N3));
+                    const uint32_t pair = q < 4 ? (uint32_t)(o1 - o0) * 16u : zeros - (slot + (uint32_t)o0 * 16u);
+                    issue(smem_desc(slot, pair, row_bytes) + (uint64_t)o0, b0 + (uint64_t)(q * 2 * N3));
                 }
             } else {
                 uint64_t ak = smem_desc(slot, (uint32_t)P * 16u, row_bytes), bk = b0;
@@ -470,10 +480,11 @@ static inline bool march_plan(int B, int D, int H, int W, int Cs, int N, bool pa
                 // with passes, a weight buffer is overwritten two passes later: the ring must not reach back
                 // that far (its slices in flight fit one pass)
                 const int last = D - (zt - 1) * Lz + (zt > 1 ? 1 : 0);
+                const int fixed = wbufs * w_bytes + (pairs ? cm_zero_bytes(nx8) : 0);
                 int stages = CM_MAX_STAGES;
                 if (passes > 1 && stages > last + 1) stages = last + 1;
-                while (stages > 2 && wbufs * w_bytes + stages * slot > CM_SMEM_LIMIT) --stages;
-                if (pieces <= CM_NE * 32 * CM_STG && wbufs * w_bytes + stages * slot <= CM_SMEM_LIMIT) {
+                while (stages > 2 && fixed + stages * slot > CM_SMEM_LIMIT) --stages;
+                if (pieces <= CM_NE * 32 * CM_STG && fixed + stages * slot <= CM_SMEM_LIMIT) {
                     const i64 tiles = (i64)B * zt * yt * xt;
                     const i64 rounds = (tiles + sms - 1) / sms;
                     const double cost = (double)rounds * march_tile_cycles(N, nx8, Lz, np, passes, pairs) *
@@ -482,7 +493,7 @@ static inline bool march_plan(int B, int D, int H, int W, int Cs, int N, bool pa
                         best_cost = cost;
                         int cols = 32;
                         while (cols < nx8 * Lz * N) cols *= 2;
-                        int smem = wbufs * w_bytes + stages * slot;
+                        int smem = fixed + stages * slot;
                         if (smem < 116 * 1024) smem = 116 * 1024;  // one block per SM (tensor memory)
                         best = MarchPlan{nx8, Lz, KC, passes, np, pieces, xt, yt, zt, stages, slot, w_bytes, wbufs,
                                          cols, smem, (int)(tiles < sms ? tiles : sms), tiles};
