@@ -616,10 +616,11 @@ static inline bool step_rows_vec(const void* p_in, const void* e, const void* p_
 }
 
 // The finest level's neighbour sum in FP64, in the reference's order, from the six neighbours' values (x + 1, x - 1,
-// y + 1, ...) and the operator bytes of the cell and its three lower neighbours: each weight is 0 or 1.
+// y + 1, ...) and the operator bytes of the cell and its three lower neighbours: each weight is 0 or 1, and the product
+// with 0 is formed in T (the weight as a double would cost a conversion a term): infinities and NaN pass as they do there.
 template <typename T>
 __device__ __forceinline__ double weighted(uint32_t o, uint32_t ox, uint32_t oy, uint32_t oz, const T* nb) {
-    auto w = [](uint32_t bit, T v) { return bit ? (double)v : 0.0; };
+    auto w = [](uint32_t bit, T v) { return (double)(bit ? v : v * T(0)); };
     return w(o & 8u, nb[0]) + w(ox & 8u, nb[1]) + w(o & 16u, nb[2]) + w(oy & 16u, nb[3]) + w(o & 32u, nb[4]) +
            w(oz & 32u, nb[5]);
 }
