@@ -1580,13 +1580,22 @@ int solve_step(const double* p64_in, const float* e, double* p64_out, const floa
     const double inv_delta2 = 1.0 / ((double)delta * (double)delta);
     const bool vec = step_rows_vec(p64_in, e, p64_out, op0, d_in, d_out, nz);
     int blocks;
-    if (g_skip_air) {
+    auto one = [&](auto kernel) {
+        launch(blocks, RN_THREADS, 0, s)(kernel, p64_in, e, p64_out, b, op0, inv_delta2, nx, ny, nz, r_out,
+                                         (double2*)partials, d_in, d_out, state);
+        return check_launch("k_step_residual");
+    };
+    if (C <= step_one_launch(MODE)) {
+        blocks = g_skip_air ? row_grid<k_step_residual<MODE, true>>(C) : clb_mg_residual_partials(C);
+        if (g_skip_air ? one(k_step_residual<MODE, true>) : one(k_step_residual<MODE, false>)) return 1;
+    } else if (g_skip_air) {
         launch(row_grid<k_step_rows<MODE, true>>(C), RN_THREADS, 0, s)(k_step_rows<MODE, true>, p64_in, e, p64_out, op0, nx,
                                                                       ny, nz, d_in, d_out, state, vec);
         CLB_LAUNCH_CHECK("k_step_rows");
         blocks = row_grid<k_residual_rows<double, true>>(C);
         launch(blocks, RN_THREADS, 0, s)(k_residual_rows<double, true>, (const double*)p64_out, b, op0, inv_delta2, nx, ny,
                                          nz, r_out, (double2*)partials);
+        CLB_LAUNCH_CHECK("k_residual_rows");
     } else {
         launch(row_grid<k_step_rows<MODE, false>>(C), RN_THREADS, 0, s)(k_step_rows<MODE, false>, p64_in, e, p64_out, op0,
                                                                        nx, ny, nz, d_in, d_out, state, vec);
@@ -1594,8 +1603,8 @@ int solve_step(const double* p64_in, const float* e, double* p64_out, const floa
         blocks = clb_mg_residual_partials(C);
         launch(blocks, RN_THREADS, 0, s)(k_residual_rows<double, false>, (const double*)p64_out, b, op0, inv_delta2, nx, ny,
                                          nz, r_out, (double2*)partials);
+        CLB_LAUNCH_CHECK("k_residual_rows");
     }
-    CLB_LAUNCH_CHECK("k_residual_rows");
     launch(1, 256, 0, s)(k_reduce_partials, (const double2*)partials, blocks, (double2*)out);
     CLB_LAUNCH_CHECK("k_reduce_partials");
     return 0;

@@ -487,20 +487,27 @@ constexpr int RN_THREADS = 256;
 // When r_out is given the residual is stored rounded to float at every cell (0 outside interior
 // fluid cells): it is the right-hand side of the next correction solve.
 //
-// The refinement and flexible-CG steps first form the new pressure cell by cell (step_rows_block), then
-// take its residual here:
+// The refinement and flexible-CG steps form the new pressure and take its residual:
 //  RES_IR:   p_out = p_in + e
 //  RES_FCG:  the search direction d = e + beta d_in (rounded to float, written to d_out) and
 //            p_out = p_in + alpha d, with alpha and beta read from state[0] and state[1] (k_fcg_scalars).
-// One pass that forms the neighbours' new pressures as it needs them reads less, but converts between float and
-// double about 34 times a cell, at an eighth of the rate of the additions. A step's launches (B200, us, cold
-// cache): six scenes of 48^3-96^3 14 + 65 (184 in one pass), 128^3 pool 27 in one pass, 256^3 block 25 + 39 (63).
-// Bound by the latency of a row's rounds of loads (two cells of a lane at a time) at 24-32 warps an SM.
+// Large grids in two launches, the pressure cell by cell (step_rows_block) and then its residual (residual_rows_block):
+// bound by the latency of a row's rounds of loads (two cells of a lane at a time) at 24-32 warps an SM. Small ones in
+// one (step_residual_block), which forms the neighbours' new pressures as it needs them: fewer bytes and a launch less, but
+// about 34 conversions between float and double a cell, at an eighth of the rate of the additions (RES_IR: 21).
+// A step with its reduction, device time (B200, us, one launch / two; liquid in all of the grid, in half of it):
+//   RES_FCG  16^3 6.7 / 8.3, 6.3 / 7.9    48^3 6.9 / 7.4, 6.5 / 7.1    64^3 8.7 / 8.9, 7.8 / 7.6    72^3 12.2 / 11.1,
+//            10.4 / 9.8    128^3 31.7 / 24.9, 20.0 / 17.4    256^3 229 / 182, 142 / 111
+//   RES_IR   48^3 6.1 / 6.9, 5.8 / 6.5    96^3 12.1 / 13.6, 11.3 / 12.8    128^3 20.1 / 21.8, 14.1 / 16.7
+//            160^3 49.1 / 47.8, 24.3 / 29.5    256^3 166 / 157, 104 / 97
+// and from the host the launch saved is 2.2 us where the GPU waits for it.
 // SKIP (refinement and FCG steps): cells that are not interior fluid cells are neither read nor
 // written. Every value there is 0 when the caller keeps the invariant (e, d_in, p_in, and the
 // outputs zeroed outside the fluid once per solve), so the outputs and sums are those of the full
 // pass; the per-lane summation order over fluid cells is unchanged.
 enum { RES_IR = 1, RES_FCG = 2 };
+// Cells up to which a step is one launch.
+__host__ __device__ constexpr i64 step_one_launch(int mode) { return mode == RES_FCG ? 300000 : 4500000; }
 
 // Whether row `base` (nz cells of the packed finest operator) holds a fluid cell, for the whole warp:
 // one 8-byte load per lane per 256 cells (when the row starts 8-byte aligned) instead of the per-cell
@@ -625,12 +632,32 @@ __device__ __forceinline__ double weighted(uint32_t o, uint32_t ox, uint32_t oy,
            w(oz & 32u, nb[5]);
 }
 
+// The sums of a block's threads to *partial.
+__device__ __forceinline__ void residual_partial(double rr, double bb, double2* __restrict__ partial) {
+    __shared__ double2 s_red[RN_THREADS / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        rr += __shfl_xor_sync(0xffffffffu, rr, o);
+        bb += __shfl_xor_sync(0xffffffffu, bb, o);
+    }
+    if (lane == 0) s_red[warp] = make_double2(rr, bb);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double2 t = s_red[0];
+        for (int q = 1; q < RN_THREADS / 32; ++q) {
+            t.x += s_red[q].x;
+            t.y += s_red[q].y;
+        }
+        *partial = t;
+    }
+}
+
 // Block `blk` of `nblk` blocks sharing the rows; its partial sums go to *partial.
 template <typename PT, bool SKIP = false>
 __device__ __forceinline__ void residual_rows_block(int blk, int nblk, const PT* p, const float* __restrict__ b,
                                                     const uint8_t* __restrict__ op0, double inv_delta2, int nx, int ny,
                                                     int nz, float* __restrict__ r_out, double2* __restrict__ partial) {
-    __shared__ double2 s_red[RN_THREADS / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int sx = ny * nz, sy = nz;
     double rr = 0.0, bb = 0.0;
@@ -696,21 +723,7 @@ __device__ __forceinline__ void residual_rows_block(int blk, int nblk, const PT*
             }
         }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        rr += __shfl_xor_sync(0xffffffffu, rr, o);
-        bb += __shfl_xor_sync(0xffffffffu, bb, o);
-    }
-    if (lane == 0) s_red[warp] = make_double2(rr, bb);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double2 t = s_red[0];
-        for (int q = 1; q < RN_THREADS / 32; ++q) {
-            t.x += s_red[q].x;
-            t.y += s_red[q].y;
-        }
-        *partial = t;
-    }
+    residual_partial(rr, bb, partial);
 }
 
 template <typename PT, bool SKIP = false>
@@ -720,6 +733,88 @@ __global__ void __launch_bounds__(RN_THREADS) k_residual_rows(const PT* p, const
                                                                double2* __restrict__ partials) {
     pdl_begin();
     residual_rows_block<PT, SKIP>(blockIdx.x, gridDim.x, p, b, op0, inv_delta2, nx, ny, nz, r_out, partials + blockIdx.x);
+}
+
+// The step and its residual in one pass, a warp per row.
+template <int MODE, bool SKIP>
+__device__ __forceinline__ void step_residual_block(int blk, int nblk, const double* __restrict__ p_in,
+                                                    const float* __restrict__ e, double* __restrict__ p_out,
+                                                    const float* __restrict__ b, const uint8_t* __restrict__ op0,
+                                                    double inv_delta2, int nx, int ny, int nz,
+                                                    float* __restrict__ r_out, double2* __restrict__ partial,
+                                                    const float* __restrict__ d_in, float* __restrict__ d_out,
+                                                    const double* __restrict__ state) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int sx = ny * nz, sy = nz;
+    double rr = 0.0, bb = 0.0;
+    double alpha = 0.0, beta = 0.0;
+    if (MODE == RES_FCG) {
+        alpha = state[0];
+        beta = state[1];
+    }
+    auto dv = [&](int q) -> float { return (float)((double)__ldg(e + q) + beta * (double)__ldg(d_in + q)); };
+    auto pv = [&](int q) -> double {
+        if (MODE == RES_IR) return (double)__ldg(p_in + q) + (double)__ldg(e + q);
+        return (double)__ldg(p_in + q) + alpha * (double)dv(q);
+    };
+    const int rows = nx * ny;
+    for (int r = blk * (RN_THREADS / 32) + warp; r < rows; r += nblk * (RN_THREADS / 32)) {
+        const int i = r / ny, j = r - i * ny;
+        const bool row_in = i >= 1 && i <= nx - 2 && j >= 1 && j <= ny - 2;
+        const int base = r * nz;
+        if (SKIP && (!row_in || !row_has_fluid(op0, base, nz, lane))) continue;
+        // a lane's operator bytes of 8 consecutive steps are loaded together, so a step waits on one
+        // round of loads (its stencil), not two (the byte that says whether the cell is fluid first)
+        for (int k0 = 0; k0 < nz; k0 += 256) {
+            unsigned long long ops = 0ull;  // byte m: the operator of step m
+#pragma unroll
+            for (int m = 0; m < 8; ++m) {
+                const int k = k0 + lane + 32 * m;
+                if (k < nz) ops |= (unsigned long long)__ldg(op0 + base + k) << (8 * m);
+            }
+#pragma unroll 1
+            for (int m = 0; m < 8; ++m) {
+                const int k = k0 + lane + 32 * m;
+                if (k >= nz) continue;
+                const int c = base + k;
+                const uint32_t o = (uint32_t)(ops >> (8 * m)) & 0xffu;
+                const bool in = row_in && k >= 1 && k <= nz - 2 && (o & 64u);
+                if (SKIP && !in) continue;
+                const double pc = pv(c);
+                p_out[c] = pc;
+                if (MODE == RES_FCG) d_out[c] = dv(c);
+                float rf = 0.0f;
+                if (in) {
+                    const uint32_t ox = __ldg(op0 + c - sx), oy = __ldg(op0 + c - sy), oz = __ldg(op0 + c - 1);
+                    const double ws = (double)bitf(o, 3) * pv(c + sx) + (double)bitf(ox, 3) * pv(c - sx) +
+                                      (double)bitf(o, 4) * pv(c + sy) + (double)bitf(oy, 4) * pv(c - sy) +
+                                      (double)bitf(o, 5) * pv(c + 1) + (double)bitf(oz, 5) * pv(c - 1);
+                    const double bv = (double)__ldg(b + c);
+                    const double res = bv - (ws - (double)(o & 7u) * pc) * inv_delta2;
+                    rr += res * res;
+                    bb += bv * bv;
+                    rf = (float)res;
+                }
+                if (r_out) r_out[c] = rf;
+            }
+        }
+    }
+    residual_partial(rr, bb, partial);
+}
+
+template <int MODE, bool SKIP>
+__global__ void __launch_bounds__(RN_THREADS) k_step_residual(const double* __restrict__ p_in,
+                                                               const float* __restrict__ e, double* __restrict__ p_out,
+                                                               const float* __restrict__ b,
+                                                               const uint8_t* __restrict__ op0, double inv_delta2,
+                                                               int nx, int ny, int nz, float* __restrict__ r_out,
+                                                               double2* __restrict__ partials,
+                                                               const float* __restrict__ d_in,
+                                                               float* __restrict__ d_out,
+                                                               const double* __restrict__ state) {
+    pdl_begin();
+    step_residual_block<MODE, SKIP>(blockIdx.x, gridDim.x, p_in, e, p_out, b, op0, inv_delta2, nx, ny, nz, r_out,
+                                    partials + blockIdx.x, d_in, d_out, state);
 }
 
 // Flexible conjugate gradients with the W-cycle as preconditioner (Notay's FCG with truncation 1;
