@@ -1133,12 +1133,19 @@ static int launch_coarse_slabs(const LevelView& v, bool along_j, int cs, float d
 // launched, 0 if the caller must go on, -1 on error. More slabs cost nothing but their ghost planes (a full level of
 // 41 x 9 x 34, us an iteration: 0.46 on 8, 0.42 on 16; of 9 x 27 x 27 0.47, 0.41, 0.38 on 4, 8, 16), one block saves
 // the cluster barrier (8 x 8 x 46: 0.25, against 0.36 to 0.40 on 2 to 8).
+// A solve of few iterations does not earn back what the one block spends on its lists and registers, 3.4 us and 1 ns a cell
+// more than k_coarse_solve, whose iterations take 0.4 us and 1.5 ns a cell longer. One, two, three, five iterations, us more
+// (+) or less than k_coarse_solve: 8 x 8 x 8 +2.6 +1.9 +1.1 -0.4, 9 x 25 x 10 +2.4 +0.1 -2.0 -6.4, 9 x 22 x 13 +2.1 -0.7
+// -3.6 -9.1. A cluster is ahead from the first (10 x 23 x 18: -1.0).
 int coarse_slabs(const LevelView& v, float delta, int iterations, cudaStream_t s) {
     if (!g_use_cluster || v.l0 || iterations < 1 || v.nx < 3 || v.ny < 3 || v.nz < 3) return 0;
     const bool along_j = v.ny > v.nx;
     const int n0 = along_j ? v.ny : v.nx, n1 = along_j ? v.nx : v.ny;
     const i64 plane = (i64)(n1 - 2) * ((v.nz - 1) / 2);  // slots of a colour in a plane
-    for (int most = plane * (n0 - 2) <= COARSE_SLAB_THREADS ? 1 : CLUSTER_MAX; most > 0; most = most > 8 ? 8 : 0) {
+    const bool single = plane * (n0 - 2) <= COARSE_SLAB_THREADS;
+    const i64 cells = (i64)(v.nx - 2) * (v.ny - 2) * (v.nz - 2);
+    if (single && iterations * (800 + 3 * cells) <= 6800 + 2 * cells) return 0;
+    for (int most = single ? 1 : CLUSTER_MAX; most > 0; most = most > 8 ? 8 : 0) {
         const int cs = most < n0 - 2 ? most : n0 - 2;
         if (plane * coarse_slab_planes(cs, n0) > COARSE_SLAB_THREADS ||
             coarse_slab_smem(cs, n0, n1, v.nz) > kBottomSmemLimit)
