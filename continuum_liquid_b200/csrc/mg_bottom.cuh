@@ -22,6 +22,7 @@
 // Cycles of a phase (B200, 25 / 256 / 512 cells of a colour): 151 / 186 / 240; with 8 warps throughout, up to two
 // cells a thread, unsplit rows and the general division 211 / 224 / 384.
 #pragma once
+#include "divide.cuh"
 #include "multigrid.cuh"
 
 namespace clb {
@@ -56,18 +57,6 @@ __device__ __forceinline__ int colour_cell(int r, int colour, int nx, int ny, in
     const int k = 1 + 2 * s + ((i + j + 1 + colour) & 1);
     if (i > nx - 2 || k > nz - 2) return -1;
     return (i * ny + j) * nz + k;
-}
-
-// x / d for a positive integer-valued d up to 32768 (every diagonal: a sum of small weights) with r = 1 / d correctly
-// rounded: Markstein's correction (P. Markstein, IBM J. Res. Dev. 34, 1990) of the product q = x r by its exact
-// remainder x - q d. Four dependent operations after x, without a branch, instead of the general division's dozen.
-// Correctly rounded for every significand and every such d (checked exhaustively) where |x| >= 2^-111; below, where
-// the remainder is no longer exact, the last bit of a subnormal quotient may differ. Infinities and NaN as x / d;
-// a zero quotient is +0.
-__device__ __forceinline__ float divide_by(float x, float d, float r) {
-    const float q = x * r;
-    const float y = __fmaf_rn(__fmaf_rn(-q, d, x), r, q);
-    return fabsf(x) < __int_as_float(0x7f800000) ? y : q;
 }
 
 // B's p in shared memory: cells of one colour together, rows of half = (nz - 1) / 2 slots (those of the
