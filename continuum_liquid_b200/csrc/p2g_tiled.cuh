@@ -19,7 +19,8 @@
 // in a fixed order: no floating-point atomics (the counts use integer shared-memory atomics, which
 // commute), and the same result on every run.
 //
-// A row's particles are one contiguous range: the warp copies it to its own buffer in shared memory with consecutive
+// A row's particles are one contiguous range: the warp copies it to its own buffer in shared memory (a longer row in equal
+// shares of its bins, as the ordered walk does: 4^3 cells of 500 particles 1330 us, 4920 in parts of the range) with consecutive
 // 16-byte loads, the next phase's row before the barrier, and the lanes read their bins there (lanes that read
 // their own bins from global memory touch 32 lines a load). The 16 warps of a block take one row each in
 // every phase. Bound by the barriers between the phases and the FP32 pipe (46 % of the issue slots: a phase lasts as
@@ -31,7 +32,12 @@
 
 namespace clb {
 
-constexpr i64 P2GT_MIN_CELLS = 3500000;  // 2.8M cells: ordered 461, tiled 518 us; 160^3: 297, 266
+// The number of particles is not known to the host here, so the line is drawn by cells. Ordered / tiled, us: full blocks
+// of 2.8M cells 461 / 518, of 160^3 297 / 266; other fillings at 160^3, 192^3 and 256^3 (uniformly random): a layer of 8 cells
+// along j 216 / 196, 303 / 284, 587 / 441, along i 163 / 131, 244 / 186, 509 / 349, along k 307 / 294, 455 / 438, 828 / 741, of 30 along
+// j 389 / 410, 542 / 554, 977 / 907; half a grid of 2 a cell 452 / 416, 742 / 661, 1634 / 1473; one clump of 32^3 cells 127 /
+// 152, 187 / 161, 334 / 206. Only very dense clumps stay with the walk (16^3 cells of 64 particles 412 / 490, 428 / 498, 504 / 506).
+constexpr i64 P2GT_MIN_CELLS = 3500000;
 constexpr int P2GT_TI = 10, P2GT_TJ = 10, P2GT_TK = 30;
 constexpr int P2GT_ROWS_I = P2GT_TI + 2, P2GT_ROWS_J = P2GT_TJ + 2;
 constexpr int P2GT_CELLS = P2GT_TI * P2GT_TJ * P2GT_TK;
@@ -114,6 +120,25 @@ __device__ __forceinline__ void p2g_tile(int tile, const float* __restrict__ pos
             }
             return skip;
         };
+        // A row of more particles than the buffer: the next ones of every bin, in equal shares of the buffer (one range of the
+        // row would be a few bins' and leave the other lanes without work). This lane's are q0 .. q1 - 1 in the buffer.
+        auto stage_shares = [&](int& q0, int& q1) {
+            const unsigned active = __ballot_sync(0xffffffffu, n > 0);
+            const int share = P2GT_ROW / __popc(active);
+            q0 = __popc(active & ((1u << lane) - 1u)) * share;
+            q1 = q0 + min(n, share);
+            for (unsigned left = active; left; left &= left - 1) {
+                const int l = __ffs(left) - 1;
+                const i64 from = 3 * (i64)__shfl_sync(0xffffffffu, begin, l);
+                const int m = __shfl_sync(0xffffffffu, q1 - q0, l), to = 3 * __shfl_sync(0xffffffffu, q0, l);
+                for (int t = lane; t < 3 * m; t += 32) {
+                    p2g_cp4(bp32 + 4 * (to + t), pos + from + t);
+                    p2g_cp4(bv32 + 4 * (to + t), vel + from + t);
+                }
+            }
+            begin += q1 - q0;
+            n -= q1 - q0;
+        };
         auto take = [&](int b, int c) {
             begin = b;
             n = c;
@@ -122,7 +147,7 @@ __device__ __forceinline__ void p2g_tile(int tile, const float* __restrict__ pos
             if (some) {
                 first = __shfl_sync(0xffffffffu, begin, __ffs(some) - 1);
                 last = __shfl_sync(0xffffffffu, begin + n, 31 - __clz(some));
-                shift = stage(first, min(P2GT_ROW, last - first));
+                if (last - first <= P2GT_ROW) shift = stage(first, last - first);
             }
         };
         {
@@ -143,18 +168,8 @@ __device__ __forceinline__ void p2g_tile(int tile, const float* __restrict__ pos
                 for (int a = 0; a < 6; ++a) vu[a] = wu[a] = vv[a] = wv[a] = vw[a] = ww[a] = 0ull;
                 const float fbx = (float)bx, fby = (float)by, fbz = (float)bz;
                 const int li = bx - i0, lj = by - j0, lk = bz - k0;
-                for (int base = first; base < last; base += P2GT_ROW) {
-                    const int m = min(P2GT_ROW, last - base);
-                    if (base > first) {
-                        __syncwarp();
-                        shift = stage(base, m);
-                    }
-                    p2g_cp_wait();
-                    __syncwarp();
-                    const float* bq = bp + shift;
-                    const float* bw = bv + shift;
-                    const int q1 = min(begin + n, base + m) - base;
-                    for (int q = max(begin, base) - base; q < q1; ++q) {
+                auto sum = [&](const float* bq, const float* bw, int q0, int q1) {
+                    for (int q = q0; q < q1; ++q) {
                         const float sx = bq[3 * q] * inv_dx, sy = bq[3 * q + 1] * inv_dx, sz = bq[3 * q + 2] * inv_dx;
                         // the reference's face positions: cell c's u face at c + 1 on x, its v and w faces
                         // at c + 0.5; here c = b - 1, b, b + 1 (full) and b, b + 1 (half)
@@ -191,6 +206,27 @@ __device__ __forceinline__ void p2g_tile(int tile, const float* __restrict__ pos
                                   ck = clampi((int)sz, 1, nz - 2) - k0;
                         if (ci >= 0 && ci < P2GT_TI && cj >= 0 && cj < P2GT_TJ && ck >= 0 && ck < P2GT_TK)
                             atomicAdd(s_cnt + (ci * P2GT_TJ + cj) * P2GT_TK + ck, 1);
+                    }
+                };
+                if (last - first > P2GT_ROW) {
+                    do {
+                        int q0, q1;
+                        stage_shares(q0, q1);
+                        p2g_cp_wait();
+                        __syncwarp();
+                        sum(bp, bv, q0, q1);
+                        __syncwarp();
+                    } while (__any_sync(0xffffffffu, n > 0));
+                } else {
+                    // Runs once: written as the loop that it would be over a longer row. Without one, lanes without particles
+                    // went on to what follows by themselves, ahead of the others, and all of it was issued twice (2
+                    // particles a bin at 160^3: 495 us, with the loop 410).
+                    for (int base = first; base < last; base += P2GT_ROW) {
+                        const int m = min(P2GT_ROW, last - base);
+                        if (base > first) __syncwarp();
+                        p2g_cp_wait();
+                        __syncwarp();
+                        sum(bp + shift, bv + shift, max(begin, base) - base, min(begin + n, base + m) - base);
                     }
                 }
                 __syncwarp();
