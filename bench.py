@@ -721,6 +721,22 @@ def pressure_error_audit(sim, snapshot, end_positions, steps, min_size):
             "replay_bit_exact": replay_exact}
 
 
+def printed_line(line):
+    """The printed line and the parts that go to stderr instead: readers of the line may keep only its last 10,000
+    characters, so the per-variant and per-step records are reduced to a time each and to their maxima."""
+    poisson, audit = line["poisson"], line["pressure_error"]
+    short = dict(line)
+    variants = {k: v for k, v in poisson.items() if isinstance(v, dict) and "ms_mean" in v and k != "timed_steps"}
+    short["poisson"] = {k: v for k, v in poisson.items() if k not in variants}
+    short["poisson"]["variants_ms"] = {k: round(v["ms_mean"], 3) for k, v in variants.items()}
+    timed = short["poisson"].get("timed_steps")
+    if isinstance(timed, dict):
+        short["poisson"]["timed_steps"] = {k: v for k, v in timed.items() if k != "history_last_step"}
+    if isinstance(audit, dict):
+        short["pressure_error"] = {k: v for k, v in audit.items() if k != "steps"}
+    return short, {"poisson": poisson, "pressure_error": audit}
+
+
 def p2g_kernel(tiled, cells):
     """The P2G kernel a step launches (csrc/p2g_tiled.cuh P2GT_MIN_CELLS, csrc/p2g_ordered.cuh P2GO_MIN_CELLS)."""
     if tiled and cells >= 3_500_000:
@@ -1203,7 +1219,9 @@ def our_arm(args):
             "clocks": clock_summary,
             "gpu_launches": int(gpu_launches),
         }
-        print(json.dumps(line), flush=True)
+        short, details = printed_line(line)
+        print(json.dumps({"details": details}), file=sys.stderr, flush=True)
+        print(json.dumps(short), flush=True)
     group.close()
 
 
