@@ -737,6 +737,11 @@ def printed_line(line):
     return short, {"poisson": poisson, "pressure_error": audit}
 
 
+def update_kernel(particles):
+    """The particle update a step launches (csrc/g2p_tiled.cuh PUT_MIN_PARTICLES)."""
+    return "k_particle_update_tiled" if particles >= 2_300_000 else "k_particle_update"
+
+
 def p2g_kernel(tiled, cells):
     """The P2G kernel a step launches (csrc/p2g_tiled.cuh P2GT_MIN_CELLS, csrc/p2g_ordered.cuh P2GO_MIN_CELLS)."""
     if tiled and cells >= 3_500_000:
@@ -796,8 +801,7 @@ def kernel_rooflines(sim, peak, ms_per_step, reps=5):
         sim.particle_work[:n].copy_(sorted_pos)
         sim.particle_velocity_work[:n].copy_(sorted_vel)
 
-    timed("particle_update", "k_particle_update_tiled (G2P, FLIP/PIC blend, advection, particle BCs)",
-          48 * n + 24 * C,
+    timed("particle_update", f"{update_kernel(n)} (G2P, FLIP/PIC blend, advection, particle BCs)", 48 * n + 24 * C,
           lambda: pm.particle_update(k, None, sim.particle_work, sim.particle_velocity_work, (sim.u, sim.v, sim.w),
                                      (sim.u_work, sim.v_work, sim.w_work), sim.obstacle, n, gs, sim.dx, sim.dt,
                                      sim.options.flip_ratio, bins=(sim.scan_outputs[0], sim.bin_counts)),

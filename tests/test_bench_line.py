@@ -39,3 +39,7 @@ def test_printed_line_is_short_and_complete():
     assert short["pressure_error"] == {"reference": "x" * 250, "rel_l2_error_max": 2e-8}
     assert details == {"poisson": line["poisson"], "pressure_error": line["pressure_error"]}
 
+
+def test_kernel_names():
+    assert bench.update_kernel(2_299_999) == "k_particle_update" and bench.update_kernel(2_300_000) == "k_particle_update_tiled"
+    assert [bench.p2g_kernel(True, c) for c in (100_000, 3_499_999, 3_500_000)] == ["k_p2g_gather", "k_p2g_ordered", "k_p2g_tiled"]
