@@ -17,31 +17,11 @@
 namespace clb {
 namespace conv {
 
-using tc::TC_KC;
 using tc::TC_M;
-using tc::TC_THREADS;
 
 struct Vol {
     int B, D, H, W;
-    __device__ __forceinline__ int voxels() const { return B * D * H * W; }
 };
-
-// neighbour of voxel (b, z, y, x) at tap t, or -1 outside the volume
-__device__ __forceinline__ int tap_neighbour(const Vol& g, int b, int z, int y, int x, int tap, int sign) {
-    const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
-    const int zz = z + sign * dz, yy = y + sign * dy, xx = x + sign * dx;
-    if (zz < 0 || zz >= g.D || yy < 0 || yy >= g.H || xx < 0 || xx >= g.W) return -1;
-    return ((b * g.D + zz) * g.H + yy) * g.W + xx;
-}
-
-__device__ __forceinline__ void decode(const Vol& g, int v, int& b, int& z, int& y, int& x) {
-    x = v % g.W;
-    int r = v / g.W;
-    y = r % g.H;
-    r /= g.H;
-    z = r % g.D;
-    b = r / g.D;
-}
 
 __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
