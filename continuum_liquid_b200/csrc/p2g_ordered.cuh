@@ -18,9 +18,10 @@
 // What bounds it: instruction issue, once the particles come from shared memory. A lane that reads its own bin's
 // particles from global memory touches 32 lines with every load, and the line rate of L1 then bounds the
 // kernel; so a warp takes a row of 32 bins along k, whose particles are one contiguous range, copies that range to
-// its own buffer with consecutive loads, and each lane walks its bin there. A row of more particles than the buffer goes in
-// rounds that give every bin an equal share of it; parts of the row's range would leave the lanes of all other bins
-// waiting for a few (4^3 cells of 500 particles each: 410 us against 1030, 16^3 of 64: 400 against 640). Blocks handle one component each:
+// its own buffer with consecutive loads, and each lane walks its bin there. A row of more particles than the buffer goes part
+// by part, or, where its bins are so full that a part is a few bins' and leaves the other lanes waiting, in rounds that give
+// every bin an equal share of the buffer (128^3, 4^3 cells of 500 particles each: 400 us, in parts 1030; 16^3 of 64: 410,
+// 640; 40^3 of 32, still in parts: 629, in shares 640 and more). Blocks handle one component each:
 // the 12 sums of a bin stay in registers at 16 warps an SM, a tile's halo is one-sided along the other axes, and
 // small grids still have enough blocks.
 //
@@ -152,6 +153,7 @@ __device__ __forceinline__ void p2g_cp_wait() { asm volatile("cp.async.wait_all;
 // A component's tile: TJ x TK cells of TI (an argument) planes. A row of bins is the 32 lanes of a warp and a plane
 // has 8 rows, one per warp: one bin below the tile along j and k, and one above along the component's axis.
 constexpr int P2GO_WARPS = 8, P2GO_THREADS = 32 * P2GO_WARPS;
+constexpr int P2GO_SHARE_COST = 32;  // what staging a round of shares costs, in particles of a lane
 constexpr int P2GO_ROW = 320;  // particles of a row staged at a time (a full row of 32 bins holds 256)
 template <int A>
 struct P2GTile {
@@ -241,7 +243,13 @@ __device__ __forceinline__ void p2g_ordered_tile(float* smem, int tile, const P2
         for (int t = lane; t < m; t += 32) p2g_cp4(bv32 + 4 * t, V + 3 * t);
         return skip;
     };
-    // A row of more particles than the buffer: the next ones of every bin, in equal shares of the buffer (one range of the
+    // A row of more particles than the buffer goes part after part of its range, which takes as long as each part's fullest
+    // bin, or in rounds of shares, which cost P2GO_SHARE_COST particles each besides the fullest bin's.
+    auto shares_pay = [&]() {
+        const int fullest = __reduce_max_sync(0xffffffffu, n), share = P2GO_ROW / __popc(__ballot_sync(0xffffffffu, n > 0));
+        return (last - first - 1) / P2GO_ROW * fullest > P2GO_SHARE_COST * ((fullest + share - 1) / share);
+    };
+    // A round: the next ones of every bin, in equal shares of the buffer (one range of the
     // row would be a few bins' and leave the other lanes without work). This lane's are q0 .. q1 - 1 in the buffer.
     auto stage_shares = [&](int& q0, int& q1) {
         const unsigned active = __ballot_sync(0xffffffffu, n > 0);
@@ -267,7 +275,7 @@ __device__ __forceinline__ void p2g_ordered_tile(float* smem, int tile, const P2
         if (some) {
             first = __shfl_sync(0xffffffffu, begin, __ffs(some) - 1);
             last = __shfl_sync(0xffffffffu, begin + n, 31 - __clz(some));
-            if (last - first <= P2GO_ROW) shift = stage(first, last - first);
+            shift = stage(first, min(P2GO_ROW, last - first));
         }
     };
     if (any) {
@@ -367,7 +375,9 @@ __device__ __forceinline__ void p2g_ordered_tile(float* smem, int tile, const P2
                         }
                     }
                 };
-                if (last - first > P2GO_ROW) {
+                if (last - first > P2GO_ROW && shares_pay()) {
+                    p2g_cp_wait();  // the part staged ahead
+                    __syncwarp();
                     do {
                         int q0, q1;
                         stage_shares(q0, q1);
@@ -377,10 +387,12 @@ __device__ __forceinline__ void p2g_ordered_tile(float* smem, int tile, const P2
                         __syncwarp();
                     } while (__any_sync(0xffffffffu, n > 0));
                 } else {
-                    // (once; see p2g_tile for the loop)
                     for (int base = first; base < last; base += P2GO_ROW) {
                         const int m = min(P2GO_ROW, last - base);
-                        if (base > first) __syncwarp();
+                        if (base > first) {
+                            __syncwarp();
+                            shift = stage(base, m);
+                        }
                         p2g_cp_wait();
                         __syncwarp();
                         sum(bp + shift, max(begin, base) - base, min(begin + n, base + m) - base);

@@ -19,8 +19,8 @@
 // in a fixed order: no floating-point atomics (the counts use integer shared-memory atomics, which
 // commute), and the same result on every run.
 //
-// A row's particles are one contiguous range: the warp copies it to its own buffer in shared memory (a longer row in equal
-// shares of its bins, as the ordered walk does: 4^3 cells of 500 particles 1330 us, 4920 in parts of the range) with consecutive
+// A row's particles are one contiguous range: the warp copies it to its own buffer in shared memory (a longer row as the
+// ordered walk does, in parts or equal shares of its bins: 4^3 cells of 500 particles 1310 us, in parts 4920) with consecutive
 // 16-byte loads, the next phase's row before the barrier, and the lanes read their bins there (lanes that read
 // their own bins from global memory touch 32 lines a load). The 16 warps of a block take one row each in
 // every phase. Bound by the barriers between the phases and the FP32 pipe (46 % of the issue slots: a phase lasts as
@@ -44,6 +44,7 @@ constexpr int P2GT_CELLS = P2GT_TI * P2GT_TJ * P2GT_TK;
 constexpr int P2GT_WARPS = 16;
 constexpr int P2GT_THREADS = 32 * P2GT_WARPS;
 // shared memory: velocity sums u, v, w; weight sums u, v, w; counts
+constexpr int P2GT_SHARE_COST = 16;               // as P2GO_SHARE_COST (a particle takes longer here)
 constexpr int P2GT_ROW = 304;                     // particles of a row staged at a time
 constexpr int P2GT_BUFFER = 6 * P2GT_ROW + 8;     // positions, velocities: each from a 16-byte boundary on
 constexpr int P2GT_PAD = P2GT_CELLS + 4;           // a spare cell after each array, for what falls outside the tile
@@ -120,7 +121,13 @@ __device__ __forceinline__ void p2g_tile(int tile, const float* __restrict__ pos
             }
             return skip;
         };
-        // A row of more particles than the buffer: the next ones of every bin, in equal shares of the buffer (one range of the
+        // A row of more particles than the buffer goes part after part of its range, which takes as long as each part's fullest
+        // bin, or in rounds of shares, which cost P2GT_SHARE_COST particles each besides the fullest bin's.
+        auto shares_pay = [&]() {
+            const int fullest = __reduce_max_sync(0xffffffffu, n), share = P2GT_ROW / __popc(__ballot_sync(0xffffffffu, n > 0));
+            return (last - first - 1) / P2GT_ROW * fullest > P2GT_SHARE_COST * ((fullest + share - 1) / share);
+        };
+        // A round: the next ones of every bin, in equal shares of the buffer (one range of the
         // row would be a few bins' and leave the other lanes without work). This lane's are q0 .. q1 - 1 in the buffer.
         auto stage_shares = [&](int& q0, int& q1) {
             const unsigned active = __ballot_sync(0xffffffffu, n > 0);
@@ -208,7 +215,7 @@ __device__ __forceinline__ void p2g_tile(int tile, const float* __restrict__ pos
                             atomicAdd(s_cnt + (ci * P2GT_TJ + cj) * P2GT_TK + ck, 1);
                     }
                 };
-                if (last - first > P2GT_ROW) {
+                if (last - first > P2GT_ROW && shares_pay()) {
                     do {
                         int q0, q1;
                         stage_shares(q0, q1);
@@ -218,12 +225,14 @@ __device__ __forceinline__ void p2g_tile(int tile, const float* __restrict__ pos
                         __syncwarp();
                     } while (__any_sync(0xffffffffu, n > 0));
                 } else {
-                    // Runs once: written as the loop that it would be over a longer row. Without one, lanes without particles
-                    // went on to what follows by themselves, ahead of the others, and all of it was issued twice (2
-                    // particles a bin at 160^3: 495 us, with the loop 410).
+                    // (without this loop, nearly always passed once, lanes without particles went on to what follows ahead of
+                    // the others, and all of it was issued twice: 2 particles a bin at 160^3 495 us, with it 410)
                     for (int base = first; base < last; base += P2GT_ROW) {
                         const int m = min(P2GT_ROW, last - base);
-                        if (base > first) __syncwarp();
+                        if (last - first > P2GT_ROW) {  // not staged ahead
+                            __syncwarp();
+                            shift = stage(base, m);
+                        }
                         p2g_cp_wait();
                         __syncwarp();
                         sum(bp + shift, bv + shift, max(begin, base) - base, min(begin + n, base + m) - base);
