@@ -454,7 +454,7 @@ static inline double march_tile_cycles(int N, int nx8, int Lz, int np, int passe
 
 // The block shape of a layer: the (columns, output slices, channels per pass) with the least estimated time
 // over the whole launch (rounds of persistent blocks times a tile's cycles) within the limits of shared memory
-// (226 KB), tensor memory (512 columns) and the staging threads' registers (8 pieces each). More columns share
+// (226 KB), tensor memory (512 columns) and the staging threads' registers (CM_NE pieces each). More columns share
 // the halo, more slices share the two extra slices a tile stages; few tiles leave SMs idle.
 static inline bool march_plan(int B, int D, int H, int W, int Cs, int N, bool pairs, int sms, MarchPlan& best) {
     double best_cost = -1.0;

@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(COARSE_SLAB_THREADS, 1)
 #pragma unroll
     for (int colour = 0; colour < 2; ++colour) {
         Cell& o = cell[colour];
-        // a thread without a cell loads some words and stores nothing
+        // a thread without a cell takes part in the barriers only
         o.c = o.n = row_plane + hz;
         o.up = o.n + 1;
         o.d2b = o.wxp = o.wxm = o.wyp = o.wym = o.wzp = o.wzm = 0.0f;

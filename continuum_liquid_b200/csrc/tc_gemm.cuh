@@ -1,7 +1,8 @@
-// BF16 GEMM core on the 5th-generation tensor cores (tcgen05), used by the 3-D convolutions of the
-// learned pressure warm start.
+// The tcgen05 building blocks of the 3-D convolutions of the learned pressure warm start (descriptors, tensor memory,
+// mbarriers, MMA issue), and a plain BF16 GEMM core that checks them: the self-test's kernel (tile_gemm); the layers
+// have kernels of their own (conv_march.cuh, conv_wgrad.cuh).
 //
-// One block of 128 threads computes a 128 x N tile of C = A * B^T (FP32 accumulation in tensor
+// In tile_gemm, one block of 128 threads computes a 128 x N tile of C = A * B^T (FP32 accumulation in tensor
 // memory). The K dimension is consumed in chunks of 64: the block's threads gather the A chunk
 // (128 x 64) and the B chunk (N x 64) into shared memory in the canonical no-swizzle core-matrix
 // layout (8 rows x 16 bytes per core matrix), one elected thread issues four

@@ -4,8 +4,8 @@
 // bit-exact against the CPU restatement.
 //
 // Bound by instruction issue (ray-triangle tests), so what counts is how few (cell, triangle) pairs are
-// tested. A block owns a brick of 8x8x8 cells and each of its warps a sub-brick of 4x4x2; a triangle
-// is tested by a warp only where it can be hit by one of that warp's rays. Two culls, both provably
+// tested. A block owns a brick of 16x8x8 cells and each of its warps two sub-bricks of 4x4x2; a triangle
+// is tested by a warp only where it can be hit by one of the sub-brick's rays. Two culls, both provably
 // without effect on the result:
 //
 //   Behind: a hit point is h = o + t*d with t > 0 and every component of d positive, so h >= o
@@ -27,9 +27,10 @@
 //   of the triangle's sheared bounding box. A brick whose sheared ray origins all lie outside that box,
 //   grown by this margin and the rounding of the comparison itself, cannot be hit.
 //
-// Measured (B200, icosphere of 5120 triangles at 128^3, radius 0.10-0.18): 0.12 ms a call, against
-// 3.4-5.1 ms with the behind cull alone on bricks of 4x4x16 (0.18 ms with 8x8x8 bricks and a division per
-// listed triangle).
+// Measured (B200, icosphere of 5120 triangles at 128^3, radius 0.10-0.18): 0.11 ms a call, against
+// 3.4-5.7 ms with the behind cull alone on bricks of 4x4x16 (0.18 ms with 8x8x8 bricks and a division per
+// listed triangle). Much of it is the set-up: every block forms the edges, determinant and box of every triangle that is
+// not behind it, and its warps then wait for the fullest (48 % of the issue slots, profiles/kernels_listed_cases.md).
 #pragma once
 #include "common.cuh"
 

@@ -377,7 +377,9 @@ int clb_mg_smooth(const clb_mg_hierarchy* h, int level, float* x, const float* r
  *            on the device); 0 launches them with ordinary stream serialisation. Identical results.
  *  option 2: 1 (default) runs each visit of the third-coarsest level, with its two bottom visits, as
  *            one launch of a thread-block cluster (up to 16 CTAs, distributed shared memory) when the
- *            three levels share their storage type and fit; 0 goes level by level. Identical
+ *            three levels share their storage type and fit, and solves a coarsest level by itself on
+ *            slabs of a cluster, or colour by colour over the whole GPU where its planes are too large
+ *            for that; 0 goes level by level and solves the coarsest level on one block. Identical
  *            results.
  *  option 3: 1 (default) lets clb_mg_ir_step and clb_mg_fcg_step skip the cells that are not
  *            interior fluid cells (neither read nor written); the caller keeps p64_out, d_out and
@@ -471,7 +473,8 @@ int clb_tc_test_gemm(const void* a, const void* b, float* c, int M, int N, int K
  *            once and read the taps as shifted windows of it.
  *  dgrad:    dx = conv^T(dy) * (mask_x > 0) (mask_x nullable), cout % 8 == 0, cin in {16,32,48,64,96}.
  *  wgrad:    dw[27*cin][cout] += sum over voxels (FP32 atomics; zero dw first), cout in {16, 32, 64};
- *            no tensor-core sum is longer than chunks_per_block chunks of 64 voxels. */
+ *            no tensor-core sum is longer than chunks_per_block chunks of 64 voxels (fewer than 8: such
+ *            sums are added up in registers first). */
 int clb_conv3d_arrange_weights(const float* w, void* wf, void* wd, int cin, int cout, int kpad, int kpad2,
                                void* stream);
 int clb_conv3d_forward(const void* x, const void* wf, const float* bias, void* y, int B, int D, int H, int W, int cin,
